@@ -166,6 +166,16 @@ int32_t prism_selftest_stream_layout_capped(uint32_t n, const uint32_t* rowptr, 
                                             uint32_t max_round_bytes, const double* in, double* out,
                                             uint32_t* record_bytes);
 
+/* Host replay of the dataflow sweep layout (the streamed kernel of sweeps whose
+ * slabs fit in shared memory), arguments as above: num_slabs slabs of at most
+ * max_slots value slots each (0: as many as 16 bits address); every index is
+ * checked, every worker's tasks are taken in order as their values become ready,
+ * and out receives the solution in the kernel's arithmetic and summation order.
+ * PRISM_ERR_UNSUPPORTED where a slab needs more slots. */
+int32_t prism_selftest_flow_layout(uint32_t n, const uint32_t* rowptr, const uint32_t* col, const double* val,
+                                   const double* diag, int32_t op, int32_t lower, int32_t precision,
+                                   uint32_t num_slabs, uint32_t max_slots, const double* in, double* out);
+
 /* The low-rank correction of an AMSED / MSLR level on a block of k <= 64
  * right-hand sides, alone on `device` with host arrays: Y += W (H o (W^T X)),
  * W column-major nrem x rank (rank <= 128), H of length rank, X and Y

@@ -80,6 +80,8 @@ _SIGS = {
     "prism_selftest_stream_layout_capped": (C.c_int32, [C.c_uint32, _u32p, _u32p, _f64p, _vp, C.c_int32, C.c_int32,
                                                         C.c_int32, C.c_uint32, C.c_uint32, C.c_uint32, _f64p,
                                                         _f64p, C.POINTER(C.c_uint32)]),
+    "prism_selftest_flow_layout": (C.c_int32, [C.c_uint32, _u32p, _u32p, _f64p, _vp, C.c_int32, C.c_int32,
+                                               C.c_int32, C.c_uint32, C.c_uint32, _f64p, _f64p]),
     "prism_selftest_stream_layout": (C.c_int32, [C.c_uint32, _u32p, _u32p, _f64p, _vp, C.c_int32, C.c_int32,
                                                  C.c_int32, C.c_uint32, C.c_uint32, _f64p, _f64p]),
     "prism_stream_sweep_order": (C.c_int32, [C.c_uint32, _u32p, _u32p, _f64p, _vp, C.c_int32, C.c_int32, C.c_int32,
@@ -244,6 +246,21 @@ def selftest_stream_layout(rowptr, col, val, in_, *, diag=None, op: int = 2, low
                                                np.ascontiguousarray(val, np.float64),
                                                d.ctypes.data if d is not None else None, op, int(lower), precision,
                                                num_ctas, rpc, np.ascontiguousarray(in_, np.float64), out))
+    return out
+
+
+def selftest_flow_layout(rowptr, col, val, in_, *, diag=None, op: int = 2, lower: bool = True, precision: int = 0,
+                         num_slabs: int = 4, max_slots: int = 0):
+    """Host replay of the dataflow sweep layout (no GPU): the sweep's solution as the kernel
+    would compute it, or raises PrismError naming the flaw."""
+    rp = np.ascontiguousarray(rowptr, np.uint32)
+    n = len(rp) - 1
+    out = np.zeros(n)
+    d = np.ascontiguousarray(diag, np.float64) if diag is not None else None
+    _check(load().prism_selftest_flow_layout(n, rp, np.ascontiguousarray(col, np.uint32),
+                                             np.ascontiguousarray(val, np.float64),
+                                             d.ctypes.data if d is not None else None, op, int(lower), precision,
+                                             num_slabs, max_slots, np.ascontiguousarray(in_, np.float64), out))
     return out
 
 

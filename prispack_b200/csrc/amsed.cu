@@ -492,7 +492,7 @@ bool AmsedPrecond::sweep_info(int sweep, uint32_t* n, uint64_t* nnz, uint32_t* v
     if (nnz) *nnz = s.entries();
     if (vbytes) *vbytes = s.fp32 ? 4 : 8;
     if (levels) *levels = s.num_levels;
-    if (kernel) *kernel = s.layout == LAYOUT_STREAM ? 3 : (s.layout == LAYOUT_SLAB ? 2 : 1);
+    if (kernel) *kernel = s.streamed() ? 3 : (s.layout == LAYOUT_SLAB ? 2 : 1);
     return true;
 }
 
@@ -500,7 +500,7 @@ bool AmsedPrecond::sweep_order(int sweep, StreamOrder& o) const {
     if (sweep < 0 || sweep >= (int)(2 * nlev_)) return false;
     const Level& L = lv_[sweep / 2];
     const DevSweep& d = (sweep & 1) ? L.upper : L.lower;
-    if (d.layout != LAYOUT_STREAM) return false;
+    if (!d.streamed()) return false;
     if (a_->fp32) {
         Sweep<float> lo, up;
         level_sweeps<float>(*a_->s32, (uint32_t)sweep / 2, lo, up);

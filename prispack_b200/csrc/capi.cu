@@ -178,6 +178,19 @@ static int stream_selftest(uint32_t n, const uint32_t* rowptr, const uint32_t* c
     return PRISM_OK;
 }
 
+template <typename Low>
+static int flow_selftest(uint32_t n, const uint32_t* rowptr, const uint32_t* col, const double* val,
+                         const double* diag, int op, bool lower, bool acc32, uint32_t slabs, uint32_t max_slots,
+                         const double* in, double* out) {
+    prism::Sweep<Low> s;
+    gather_sweep<Low>(n, rowptr, col, val, diag, op, lower, s);
+    prism::FlowLayout L;
+    if (!prism::flow_layout<Low>(s, prism::slab_ranges<Low>(s, slabs), max_slots ? max_slots : 0xFFFFu, L))
+        return fail(PRISM_ERR_UNSUPPORTED, "a slab needs more value slots");
+    const std::string why = prism::flow_layout_replay<Low>(s, L, acc32, in, out);
+    return why.empty() ? PRISM_OK : fail(PRISM_ERR_ARG, "dataflow layout: " + why);
+}
+
 extern "C" {
 
 const char* prism_last_error(void) { return g_last_error.c_str(); }
@@ -195,6 +208,22 @@ int32_t prism_selftest_wait_timeout(int32_t device, uint64_t wait_ns, int32_t* d
         prism::selftest_wait_timeout(device, wait_ns, &s);
         *device_status = s;
         return PRISM_OK;
+    });
+}
+
+int32_t prism_selftest_flow_layout(uint32_t n, const uint32_t* rowptr, const uint32_t* col, const double* val,
+                                   const double* diag, int32_t op, int32_t lower, int32_t precision,
+                                   uint32_t num_slabs, uint32_t max_slots, const double* in, double* out) {
+    if (!rowptr || !col || !val || !in || !out || n == 0) return fail(PRISM_ERR_ARG, "null array or empty sweep");
+    if (op < 0 || op > 3 || (op != 2 && !diag)) return fail(PRISM_ERR_ARG, "bad op / missing diagonal");
+    if (!valid_precision(precision) || num_slabs == 0) return fail(PRISM_ERR_ARG, "bad precision or slab count");
+    return guarded([&]() -> int {
+        int rc = check_gather_form(n, rowptr, col, lower);
+        if (rc) return rc;
+        if (precision == PRISM_FP64)
+            return flow_selftest<double>(n, rowptr, col, val, diag, op, lower != 0, false, num_slabs, max_slots, in, out);
+        return flow_selftest<float>(n, rowptr, col, val, diag, op, lower != 0, precision == PRISM_FP32_APPLY, num_slabs,
+                                    max_slots, in, out);
     });
 }
 

@@ -339,7 +339,24 @@ template <typename Low>
 void build_map(const DevSweep& d, const Sweep<Low>& s, const Sweep<double>& idx, SweepValueMap& M, cudaStream_t st) {
     std::vector<uint32_t> cd, cs, dd, ds;
     const bool has_diag = s.op != SWEEP_NONE;
-    if (d.layout == LAYOUT_STREAM) {
+    if (d.layout == LAYOUT_FLOW) {
+        FlowLayout F;
+        std::vector<uint32_t> cmap;
+        if (!flow_layout<Low>(s, slab_ranges<Low>(s, d.str_ctas_req), d.str_slots, F, nullptr, &cmap))
+            throw Error(PRISM_ERR_CUDA, "dataflow layout could not be rebuilt");
+        cd.reserve(cmap.size() / 2);
+        cs.reserve(cmap.size() / 2);
+        for (size_t t = 0; t < cmap.size(); t += 2) {
+            cd.push_back(cmap[t]);
+            cs.push_back((uint32_t)idx.val[cmap[t + 1]]);
+        }
+        if (has_diag) {
+            for (uint32_t p = 0; p < idx.n; ++p) {
+                dd.push_back(F.dg_pos[idx.order[p]]);
+                ds.push_back((uint32_t)idx.diag[p]);
+            }
+        }
+    } else if (d.layout == LAYOUT_STREAM) {
         StreamLayout L;
         std::vector<uint32_t> cmap;
         std::string why;
@@ -392,27 +409,29 @@ void apply_map(const Handle& h, cudaStream_t st, DevSweep& d, const SweepValueMa
                const double* D, bool ic, unsigned* bad) {
     if (!d.n) return;
     if (M.ncoef) {
-        const bool stream = d.layout == LAYOUT_STREAM;
-        Low* dst = stream ? reinterpret_cast<Low*>(d.str_blob.get())
+        const bool stream = d.streamed();
+        DevBuf<unsigned char>& blob = d.layout == LAYOUT_FLOW ? d.fl_chunks : d.str_blob;
+        Low* dst = stream ? reinterpret_cast<Low*>(blob.get())
                           : (std::is_same<Low, float>::value ? reinterpret_cast<Low*>(d.val32.get())
                                                              : reinterpret_cast<Low*>(d.val64.get()));
-        const uint64_t dst_n = stream ? d.str_blob.size() / sizeof(Low)
+        const uint64_t dst_n = stream ? blob.size() / sizeof(Low)
                                       : (std::is_same<Low, float>::value ? d.val32.size() : d.val64.size());
         k_rf_coef<Low><<<rf_grid(h, M.ncoef), kBlock, 0, st>>>(M.ncoef, M.cdst.get(), M.csrc.get(), lt, lt_n, dst,
                                                                dst_n, bad);
         PRISM_LAUNCHED();
     }
     if (M.ndiag) {
-        const int recip = d.layout == LAYOUT_STREAM && (d.op == SWEEP_DIV || d.op == SWEEP_PREDIV);
+        const int recip = d.streamed() && (d.op == SWEEP_DIV || d.op == SWEEP_PREDIV);
         const uint64_t src_n = ic ? lt_n : d.n;
-        if (d.layout == LAYOUT_STREAM && d.acc32) {
+        DevBuf<unsigned char>& blob = d.layout == LAYOUT_FLOW ? d.fl_dg : d.str_blob;
+        if (d.streamed() && d.acc32) {
             k_rf_diag<Low, float><<<rf_grid(h, M.ndiag), kBlock, 0, st>>>(
-                M.ndiag, M.ddst.get(), M.dsrc.get(), lt, D, src_n, ic, recip,
-                reinterpret_cast<float*>(d.str_blob.get()), d.str_blob.size() / sizeof(float), bad + 1);
+                M.ndiag, M.ddst.get(), M.dsrc.get(), lt, D, src_n, ic, recip, reinterpret_cast<float*>(blob.get()),
+                blob.size() / sizeof(float), bad + 1);
         } else {
-            const bool stream = d.layout == LAYOUT_STREAM;
-            double* dst = stream ? reinterpret_cast<double*>(d.str_blob.get()) : d.diag.get();
-            const uint64_t dst_n = stream ? d.str_blob.size() / sizeof(double) : d.diag.size();
+            const bool stream = d.streamed();
+            double* dst = stream ? reinterpret_cast<double*>(blob.get()) : d.diag.get();
+            const uint64_t dst_n = stream ? blob.size() / sizeof(double) : d.diag.size();
             k_rf_diag<Low, double><<<rf_grid(h, M.ndiag), kBlock, 0, st>>>(M.ndiag, M.ddst.get(), M.dsrc.get(), lt,
                                                                             D, src_n, ic, recip, dst, dst_n, bad + 1);
         }

@@ -9,6 +9,7 @@
 #include "kernels.cuh"
 #include "solve.cuh"
 #include "stream_sweep.cuh"
+#include "flow_sweep.cuh"
 
 namespace prism {
 
@@ -23,6 +24,12 @@ constexpr int kSpmvSubG = 8;                           // lanes per row in k_spm
 constexpr int kSpmvG = 1, kSpmvU = 2;                  // k_spmv: lanes per row, rows per group and pass
 // the shapes A's SpMV may take (lanes per row, rows per group and pass): one lane per row
 // suits short rows such as stencils, a group of lanes per row longer ones
+// Rows of a dataflow slab the tuner tries.  More slabs share a wavefront's rows among more SMs
+// and let a CTA take its next slab while the wavefront is elsewhere; fewer pay fewer hand-overs
+// from slab to slab (about 1 us each).  Measured (us an M^-1 apply, 1024 / 2048 / 4096 rows):
+// IC 512^2 FP64 1590 / 1269 / 1052, IC 40^3 FP64 437 / 473 / 580, AMSED 128^3 with float
+// arithmetic 4971 / 4476 / 5649.
+constexpr uint32_t kFlowSlabRows[3] = {1024, 2048, 4096};
 constexpr int kSpmvShapes = 6;
 constexpr int kSpmvShapeG[kSpmvShapes] = {1, 1, 2, 4, 8, 16};
 constexpr int kSpmvShapeU[kSpmvShapes] = {2, 4, 2, 1, 1, 1};
@@ -86,8 +93,35 @@ static void* stream_kernel(bool fp32, int op, bool acc32) {
     }
 }
 
+// acc32 as above; entries: E of the layout
+template <typename Low, typename Acc, int E>
+static void* flow_kernel_of(int op) {
+    switch (op) {
+        case SWEEP_DIV: return (void*)k_sweep_flow<Low, OP_DIV, Acc, E>;
+        case SWEEP_MUL: return (void*)k_sweep_flow<Low, OP_MUL, Acc, E>;
+        case SWEEP_NONE: return (void*)k_sweep_flow<Low, OP_NONE, Acc, E>;
+        default: return (void*)k_sweep_flow<Low, OP_PREDIV, Acc, E>;
+    }
+}
+static void* flow_kernel(bool fp32, int op, bool acc32, uint32_t entries) {
+    if (entries == 4) {
+        if (acc32) return flow_kernel_of<float, float, 4>(op);
+        return fp32 ? flow_kernel_of<float, double, 4>(op) : flow_kernel_of<double, double, 4>(op);
+    }
+    if (acc32) return flow_kernel_of<float, float, 8>(op);
+    return fp32 ? flow_kernel_of<float, double, 8>(op) : flow_kernel_of<double, double, 8>(op);
+}
+
 void launch_sweep_prepare(const Handle& h, cudaStream_t st, const DevSweep& s, const double* in, double* out) {
     if (!s.n) return;
+    if (s.layout == LAYOUT_FLOW) {
+        if (s.paired) {
+            k_flow_pair_rhs<<<vec_grid(h, s.n), kBlock, 0, st>>>(s.n, s.pair_ptr.get(), s.pair_dep.get(),
+                                                                s.pair_coef.get(), in, s.pair_rhs.get());
+            PRISM_LAUNCHED();
+        }
+        return;
+    }
     if (s.layout != LAYOUT_STREAM) {
         launch_fill(st, h, s.n, out);
         return;
@@ -120,6 +154,28 @@ void launch_sweep_prepare(const Handle& h, cudaStream_t st, const DevSweep& s, c
 
 void launch_sweep_kernel(const Handle& h, cudaStream_t st, const DevSweep& s, const double* in, double* out) {
     if (!s.n) return;
+    if (s.layout == LAYOUT_FLOW) {
+        FlowArgs a;
+        a.chunks = s.fl_chunks.get();
+        a.hdr = reinterpret_cast<const uint4*>(s.fl_hdr.get());
+        a.dg = s.fl_dg.get();
+        a.warp = reinterpret_cast<const uint4*>(s.fl_warp.get());
+        a.halo_ptr = s.fl_halo_ptr.get();
+        a.halo = reinterpret_cast<const uint2*>(s.fl_halo.get());
+        a.xch = s.fl_xch.get();
+        a.ctl = s.fl_ctl.get();
+        a.in = s.paired ? s.pair_rhs.get() : in;
+        a.out = out;
+        a.status = h.status.get();
+        a.wait_ns = kWaitNs;
+        a.slabs = s.fl_slabs;
+        a.slots = s.str_slots;
+        void* args[] = {&a};
+        PRISM_CUDA(cudaLaunchCooperativeKernel(flow_kernel(s.fp32, s.op, s.acc32, s.fl_entries), dim3(s.str_ctas), dim3(kFlowThreads),
+                                               args, s.str_smem, st));
+        PRISM_LAUNCHED();
+        return;
+    }
     if (s.layout == LAYOUT_STREAM) {
         (void)in;
         StreamArgs a;
@@ -195,7 +251,7 @@ void launch_sweep_kernel(const Handle& h, cudaStream_t st, const DevSweep& s, co
 }
 
 void launch_sweep(const Handle& h, cudaStream_t st, const DevSweep& s, const double* in, double* out) {
-    if (s.layout == LAYOUT_STREAM) launch_sweep_prepare(h, st, s, in, out);
+    if (s.streamed()) launch_sweep_prepare(h, st, s, in, out);
     launch_sweep_kernel(h, st, s, in, out);
 }
 
@@ -302,12 +358,20 @@ void init_device_info(DeviceInfo& info, int device) {
         info.stream_pair = v < 0 ? 0 : (v > 2 ? 2 : v);
     }
     if (info.stream_min_rows < 32) info.stream_min_rows = 32;
+    if (const char* e = std::getenv("PRISM_FLOW_ROWS")) info.flow_rows = (uint32_t)std::max(32, std::atoi(e));
     for (bool f32 : {false, true})
         for (int op = 0; op < 4; ++op) {
             PRISM_CUDA(cudaFuncSetAttribute(slab_kernel(f32, op), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             info.max_smem_optin));
             PRISM_CUDA(cudaFuncSetAttribute(stream_kernel(f32, op, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             info.max_smem_optin));
+            for (uint32_t e : {4u, 8u}) {
+                PRISM_CUDA(cudaFuncSetAttribute(flow_kernel(f32, op, false, e), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                info.max_smem_optin));
+                if (f32)
+                    PRISM_CUDA(cudaFuncSetAttribute(flow_kernel(true, op, true, e),
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, info.max_smem_optin));
+            }
             if (f32)
                 PRISM_CUDA(cudaFuncSetAttribute(stream_kernel(true, op, true),
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, info.max_smem_optin));
@@ -422,7 +486,10 @@ void DevSweep::release() {
     str_ctas = str_ring = str_meta_slots = str_slots = str_rounds = str_smem = 0;
     str_nnz = 0;
     str_round_cap = 0;
-    pair_ptr.release(); pair_dep.release(); pair_coef.release();
+    fl_chunks.release(); fl_dg.release(); fl_xch.release();
+    fl_hdr.release(); fl_warp.release(); fl_halo_ptr.release(); fl_halo.release(); fl_ctl.release();
+    fl_slabs = 0;
+    pair_ptr.release(); pair_dep.release(); pair_coef.release(); pair_rhs.release();
     paired = false;
     n = num_levels = 0;  // empty: nothing launches on a released sweep
 }
@@ -487,6 +554,39 @@ StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc
 template StreamPlan plan_stream<double>(const Sweep<double>&, const DeviceInfo&, bool, bool);
 template StreamPlan plan_stream<float>(const Sweep<float>&, const DeviceInfo&, bool, bool);
 
+template <typename Low>
+StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows) {
+    StreamPlan P;
+    const uint32_t nn = sweep.n;
+    if (nn == 0) return P;
+    Sweep<Low> ps;
+    if (pair) pair_sweep<Low>(sweep, ps, P.pm);
+    const Sweep<Low>& s0 = pair ? ps : sweep;
+    P.a32 = acc32 && std::is_same<Low, float>::value;
+    P.slot_bytes = P.a32 ? 4 : 8;
+    const uint32_t cap = ((uint32_t)info.max_smem_optin - flow_smem(0, P.slot_bytes)) / P.slot_bytes;
+    // A slab whose rows and halo do not fit in shared memory is split further.
+    uint32_t want = std::max(1u, (nn + rows - 1) / rows);
+    for (;; want *= 2) {
+        const std::vector<uint32_t> start = slab_ranges<Low>(s0, want);
+        if (flow_layout<Low>(s0, start, cap, P.F)) break;
+        if (nn / want < 64) return P;
+    }
+    P.ok = P.flow = true;
+    P.paired = pair;
+    P.fp32 = std::is_same<Low, float>::value;
+    P.n = s0.n;
+    P.num_levels = s0.num_levels;
+    P.op = s0.op;
+    P.ctas_req = want;
+    P.ctas = std::min(P.F.slabs, (uint32_t)info.sms);
+    P.smem = flow_smem(P.F.slots, P.slot_bytes);
+    P.nnz = s0.val.size();
+    return P;
+}
+template StreamPlan plan_flow<double>(const Sweep<double>&, const DeviceInfo&, bool, bool, uint32_t);
+template StreamPlan plan_flow<float>(const Sweep<float>&, const DeviceInfo&, bool, bool, uint32_t);
+
 void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
     const StreamLayout& L = P.L;
     release();
@@ -495,17 +595,54 @@ void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
     op = P.op;
     fp32 = P.fp32;
     acc32 = P.a32;
-    layout = LAYOUT_STREAM;
     str_ctas = P.ctas;
     str_ctas_req = P.ctas_req;
+    str_nnz = P.nnz;
+    str_smem = P.smem;
+    if (P.paired) {
+        paired = true;
+        pair_ptr.upload(P.pm.ptr.data(), P.pm.ptr.size(), st);
+        pair_dep.upload(P.pm.dep.data(), P.pm.dep.size(), st);
+        pair_coef.upload(P.pm.coef.data(), P.pm.coef.size(), st);
+        if (pair_dep.size() == 0) pair_dep.alloc(1);  // valid pointers for the prep
+        if (pair_coef.size() == 0) pair_coef.alloc(1);
+    }
+    if (P.flow) {
+        const FlowLayout& F = P.F;
+        layout = LAYOUT_FLOW;
+        fl_slabs = F.slabs;
+        str_slots = F.slots;
+        fl_entries = F.entries;
+        fl_chunks.alloc(F.chunks.size() + kFlowPad);  // the kernel brings lines past the end into L2
+        fl_chunks.upload(F.chunks.data(), F.chunks.size(), st);
+        fl_hdr.upload(F.hdr.data(), F.hdr.size(), st);
+        fl_warp.upload(F.warp.data(), F.warp.size(), st);
+        fl_halo_ptr.upload(F.halo_ptr.data(), F.halo_ptr.size(), st);
+        fl_halo.upload(F.halo.data(), F.halo.size(), st);
+        if (fl_halo.size() == 0) fl_halo.alloc(2);
+        std::vector<float> dgf;
+        if (acc32) {
+            dgf.assign(F.dg.begin(), F.dg.end());
+            fl_dg.upload(reinterpret_cast<const unsigned char*>(dgf.data()), dgf.size() * sizeof(float), st);
+        } else {
+            fl_dg.upload(reinterpret_cast<const unsigned char*>(F.dg.data()), F.dg.size() * sizeof(double), st);
+        }
+        // epoch 0 everywhere: the first sweep is epoch 1
+        fl_xch.alloc((size_t)std::max(F.published, 1u) * (acc32 ? sizeof(FlowWord<float>) : sizeof(FlowWord<double>)));
+        PRISM_CUDA(cudaMemsetAsync(fl_xch.get(), 0, fl_xch.size(), st));
+        fl_ctl.alloc(2);
+        PRISM_CUDA(cudaMemsetAsync(fl_ctl.get(), 0, 2 * sizeof(uint32_t), st));
+        if (paired) pair_rhs.alloc(n);
+        PRISM_CUDA(cudaStreamSynchronize(st));
+        return;
+    }
+    layout = LAYOUT_STREAM;
     str_slot_bytes = P.slot_bytes;
     str_round_cap = P.cap;
     str_ring = P.ring;
     str_meta_slots = L.max_rounds_per_cta;
     str_slots = L.slots;
     str_rounds = L.num_rounds;
-    str_smem = P.smem;
-    str_nnz = P.nnz;
     str_blob.upload(L.blob.data(), L.blob.size(), st);
     str_meta.upload(L.meta.data(), L.meta.size(), st);
     str_cta_round.upload(L.cta_round.data(), L.cta_round.size(), st);
@@ -516,21 +653,14 @@ void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
     str_halo_sw.upload(L.halo_sw.data(), L.halo_sw.size(), st);
     if (str_halo_row.size() == 0) str_halo_row.alloc(1);  // valid pointers for the kernel
     if (str_halo_sw.size() == 0) str_halo_sw.alloc(1);
-    if (P.paired) {
-        paired = true;
-        pair_ptr.upload(P.pm.ptr.data(), P.pm.ptr.size(), st);
-        pair_dep.upload(P.pm.dep.data(), P.pm.dep.size(), st);
-        pair_coef.upload(P.pm.coef.data(), P.pm.coef.size(), st);
-        if (pair_dep.size() == 0) pair_dep.alloc(1);  // valid pointers for the prep
-        if (pair_coef.size() == 0) pair_coef.alloc(1);
-    }
     PRISM_CUDA(cudaStreamSynchronize(st));
 }
 
 template <typename Low>
 bool DevSweep::upload(const Sweep<Low>& sweep, const DeviceInfo& info, int lay, cudaStream_t st, bool pair) {
-    if (lay == LAYOUT_STREAM) {
-        StreamPlan P = plan_stream<Low>(sweep, info, acc32, pair);
+    if (lay == LAYOUT_STREAM || lay == LAYOUT_FLOW) {
+        StreamPlan P = lay == LAYOUT_FLOW ? plan_flow<Low>(sweep, info, acc32, pair, info.flow_rows ? info.flow_rows : kFlowSlabRows[0])
+                                          : plan_stream<Low>(sweep, info, acc32, pair);
         if (!P.ok) return false;
         commit_stream(std::move(P), st);
         return true;
@@ -586,14 +716,18 @@ uint32_t stream_slab_count(uint32_t n, uint32_t num_ctas, uint32_t min_rows) {
 
 template <typename Low>
 bool DevSweep::stream_order(const Sweep<Low>& sweep, StreamOrder& o) const {
-    if (layout != LAYOUT_STREAM || sweep.n != n) return false;
+    if (!streamed() || sweep.n != n) return false;
     Sweep<Low> ps;
     PairMap pm;
     if (paired) pair_sweep<Low>(sweep, ps, pm);
     const Sweep<Low>& s = paired ? ps : sweep;
     StreamLayout L;
+    FlowLayout F;
     std::string why;
-    if (!stream_layout<Low>(s, slab_ranges<Low>(s, str_ctas_req), kNoSlot, str_slot_bytes, L, &why, &o, nullptr,
+    if (layout == LAYOUT_FLOW) {
+        if (!flow_layout<Low>(s, slab_ranges<Low>(s, str_ctas_req), str_slots, F, &o))
+            throw Error(PRISM_ERR_CUDA, "dataflow layout could not be rebuilt");
+    } else if (!stream_layout<Low>(s, slab_ranges<Low>(s, str_ctas_req), kNoSlot, str_slot_bytes, L, &why, &o, nullptr,
                             str_round_cap))
         throw Error(PRISM_ERR_CUDA, "streamed layout could not be rebuilt: " + why);
     if (paired) {
@@ -631,9 +765,10 @@ template void stream_sweep_run<double>(int, const Sweep<double>&, bool, uint32_t
 template void stream_sweep_run<float>(int, const Sweep<float>&, bool, uint32_t, const double*, double*);
 
 // Sweep-kernel autotuner: uploads the sweep in each device layout in turn
-// (level order for k_sweep, slabs for k_sweep_slab, streamed rounds for
-// k_sweep_stream), times a few launches of each, output marking included, on
-// a fixed right-hand side with CUDA events, and keeps the fastest.  Which
+// (level order for k_sweep, slabs for k_sweep_slab, dataflow slabs for k_sweep_flow
+// or, where they do not fit, rounds for k_sweep_stream), times a few launches of
+// each, output marking included, on a fixed right-hand side with CUDA events, and
+// keeps the fastest.  Which
 // kernel wins depends on how many rows a wavefront holds and how far
 // dependencies reach.
 template <typename Low>
@@ -648,22 +783,37 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
         d.upload(s, h.info, LAYOUT_LEVEL, h.stream);
         return;
     }
-    // candidates: {layout, paired}.  Single-precision arithmetic: only the streamed kernel
-    // has it (the other layouts, where the streamed one does not fit, compute in double).
-    std::vector<std::pair<int, bool>> cand;
+    // candidates.  Single-precision arithmetic: only the streamed kernels have it (the other
+    // layouts, where no streamed one fits, compute in double).  The streamed kernel is the
+    // dataflow one; the rounds take the sweeps that do not fit it.
+    struct Cand {
+        int layout;
+        bool paired;
+        uint32_t rows;
+    };
+    std::vector<Cand> cand;
+    auto streamed = [&](bool paired) {
+        if (h.info.flow_rows) {
+            cand.push_back({LAYOUT_FLOW, paired, h.info.flow_rows});
+            return;
+        }
+        for (uint32_t rows : kFlowSlabRows)  // small sweeps: one size, the others are within 3% (64^2: 151-152 us)
+            if (rows == kFlowSlabRows[0] || s.n > 16 * kFlowSlabRows[0]) cand.push_back({LAYOUT_FLOW, paired, rows});
+    };
     if (pp && h.info.stream_pair == 2) {  // paired where it fits
-        cand.push_back({LAYOUT_STREAM, true});
+        streamed(true);
     } else if (d.acc32 || mode == 3) {
-        cand.push_back({LAYOUT_STREAM, false});
-        if (pp) cand.push_back({LAYOUT_STREAM, true});
+        streamed(false);
+        if (pp) streamed(true);
     } else if (mode != 0) {
-        cand.push_back({mode == 2 ? LAYOUT_SLAB : LAYOUT_LEVEL, false});
+        cand.push_back({mode == 2 ? LAYOUT_SLAB : LAYOUT_LEVEL, false, 0});
     } else {
-        cand = {{LAYOUT_LEVEL, false}, {LAYOUT_SLAB, false}, {LAYOUT_STREAM, false}};
-        if (pp) cand.push_back({LAYOUT_STREAM, true});
+        cand = {{LAYOUT_LEVEL, false, 0}, {LAYOUT_SLAB, false, 0}};
+        streamed(false);
+        if (pp) streamed(true);
     }
-    if (cand.size() == 1) {
-        if (!d.upload(s, h.info, cand[0].first, h.stream, cand[0].second)) d.upload(s, h.info, LAYOUT_LEVEL, h.stream);
+    if (cand.size() == 1 && cand[0].layout != LAYOUT_FLOW) {
+        d.upload(s, h.info, cand[0].layout, h.stream);
         return;
     }
     DevBuf<double> in(s.n), out(s.n);
@@ -678,19 +828,24 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
     // the streamed candidates' host layouts are built concurrently
     std::vector<std::future<StreamPlan>> plans(cand.size());
     for (int c = 0; c < (int)cand.size(); ++c)
-        if (cand[c].first == LAYOUT_STREAM) {
-            const bool pc = cand[c].second, a32 = d.acc32;
-            plans[c] = std::async(std::launch::async, [&s, &h, a32, pc] { return plan_stream<Low>(s, h.info, a32, pc); });
+        if (cand[c].layout == LAYOUT_FLOW) {
+            const bool a32 = d.acc32, first = cand[c].rows == kFlowSlabRows[0] || h.info.flow_rows != 0;
+            const Cand cc = cand[c];
+            plans[c] = std::async(std::launch::async, [&s, &h, a32, cc, first] {
+                StreamPlan P = plan_flow<Low>(s, h.info, a32, cc.paired, cc.rows);
+                if (!P.ok && first) P = plan_stream<Low>(s, h.info, a32, cc.paired);
+                return P;
+            });
         }
     DevSweep kept;  // the fastest candidate so far, kept uploaded
     for (int c = 0; c < (int)cand.size(); ++c) {
         DevSweep t;
         t.acc32 = d.acc32;
-        if (cand[c].first == LAYOUT_STREAM) {
+        if (cand[c].layout == LAYOUT_FLOW) {
             StreamPlan P = plans[c].get();
             if (!P.ok) continue;
             t.commit_stream(std::move(P), h.stream);
-        } else if (!t.upload(s, h.info, cand[c].first, h.stream, cand[c].second)) {
+        } else if (!t.upload(s, h.info, cand[c].layout, h.stream)) {
             continue;
         }
         float tot = 0.f;
@@ -760,7 +915,7 @@ bool TriangularPrecond::run_sweep(cudaStream_t st, int sweep, const double* in, 
 bool TriangularPrecond::sweep_info(int sweep, uint32_t* n, uint64_t* nnz, uint32_t* vbytes, uint32_t* levels,
                                    uint32_t* kernel) const {
     const DevSweep& s = sweep == 0 ? lower_ : upper_;
-    if (kernel) *kernel = s.layout == LAYOUT_STREAM ? 3 : (s.layout == LAYOUT_SLAB ? 2 : 1);
+    if (kernel) *kernel = s.streamed() ? 3 : (s.layout == LAYOUT_SLAB ? 2 : 1);
     if (n) *n = s.n;
     if (nnz) *nnz = s.entries();
     if (vbytes) *vbytes = s.fp32 ? 4 : 8;

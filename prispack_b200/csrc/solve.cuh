@@ -9,6 +9,7 @@
 
 #include "../../include/prism_solve.h"
 #include "device_common.cuh"
+#include "flow_layout.hpp"
 #include "host_setup.hpp"
 #include "amsed_setup.hpp"
 
@@ -24,6 +25,7 @@ struct DeviceInfo {
     uint32_t slab_min_rows = 2048; // smallest slab (small systems use fewer CTAs)
     uint32_t slab_max_rows = 1u << 30;  // largest slab (default: what shared memory holds)
     uint32_t stream_min_rows = 1024;    // smallest streamed slab (small systems use fewer CTAs)
+    uint32_t flow_rows = 0;             // rows of a dataflow slab (0: the tuner's choice)
     int stream_pair = 1;           // where asked: 0 never paired, 1 the tuner decides, 2 paired (pair_sweep)
 };
 
@@ -57,14 +59,16 @@ struct DeviceCsr {
 };
 
 // Device layouts of a triangular sweep.
-enum SweepLayout : int { LAYOUT_LEVEL = 0, LAYOUT_SLAB = 1, LAYOUT_STREAM = 2 };
+enum SweepLayout : int { LAYOUT_LEVEL = 0, LAYOUT_SLAB = 1, LAYOUT_STREAM = 2, LAYOUT_FLOW = 3 };
 
 // One triangular sweep resident on the device (see build_sweep for the layout).
 // The host part of a streamed upload (pairing, layout, launch shape; no CUDA calls), which
-// DevSweep::commit_stream uploads.  ok false: the sweep does not fit the streamed layout.
+// DevSweep::commit_stream uploads: the dataflow layout F (flow) or the rounds L.
+// ok false: the sweep does not fit.
 struct StreamPlan {
-    bool ok = false, paired = false, fp32 = false, a32 = false;
+    bool ok = false, paired = false, fp32 = false, a32 = false, flow = false;
     StreamLayout L;
+    FlowLayout F;
     PairMap pm;
     uint32_t n = 0, num_levels = 0;
     int op = 0;
@@ -73,6 +77,9 @@ struct StreamPlan {
 };
 template <typename Low>
 StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair);
+// rows: of a slab (fewer where a slab's rows and halo do not fit in shared memory)
+template <typename Low>
+StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows);
 
 struct DevSweep {
     uint32_t n = 0, num_levels = 0;
@@ -93,20 +100,26 @@ struct DevSweep {
     DevBuf<uint32_t> str_halo_ptr, str_halo_row, str_halo_sw;
     uint32_t str_ctas_req = 0, str_slot_bytes = 0;  // what the layout was built with (for its export)
     uint32_t str_round_cap = 0;                     // ... and its record cap (0: none)
-    // LAYOUT_STREAM built from the paired sweep (pair_sweep): the right-hand side map the prep
-    // applies before the kernel
+    // LAYOUT_FLOW (k_sweep_flow): see FlowLayout; str_ctas_req slabs, str_slots, str_smem and
+    // str_nnz as above
+    uint32_t fl_slabs = 0, fl_entries = 0;
+    DevBuf<unsigned char> fl_chunks, fl_dg, fl_xch;
+    DevBuf<uint32_t> fl_hdr, fl_warp, fl_halo_ptr, fl_halo, fl_ctl;
+    // LAYOUT_STREAM or LAYOUT_FLOW built from the paired sweep (pair_sweep): the right-hand side
+    // map the prep applies before the kernel (LAYOUT_FLOW: into pair_rhs)
     bool paired = false;
     DevBuf<uint32_t> pair_ptr, pair_dep;
-    DevBuf<double> pair_coef;
+    DevBuf<double> pair_coef, pair_rhs;
     // Uploads the sweep in the given layout; false (nothing uploaded) when the
     // layout does not fit the sweep (stream layout only).  pair: the streamed layout
     // of the paired sweep (half the wavefronts; other layouts ignore it).
     template <typename Low>
     bool upload(const Sweep<Low>& s, const DeviceInfo& info, int layout, cudaStream_t st, bool pair = false);
     void commit_stream(StreamPlan&& plan, cudaStream_t st);
-    // the stream layout marks its own output pending; the others need launch_fill first
-    bool self_filling() const { return layout == LAYOUT_STREAM; }
-    uint64_t entries() const { return layout == LAYOUT_STREAM ? str_nnz : (fp32 ? val32.size() : val64.size()); }
+    bool streamed() const { return layout == LAYOUT_STREAM || layout == LAYOUT_FLOW; }
+    // the streamed layouts mark their own output pending or need no mark; the others need launch_fill first
+    bool self_filling() const { return streamed(); }
+    uint64_t entries() const { return streamed() ? str_nnz : (fp32 ? val32.size() : val64.size()); }
     void release();                // frees the arrays; n = 0 afterwards
     // the summation order of the streamed layout this sweep was uploaded with (s = the same
     // host sweep); false for the other layouts

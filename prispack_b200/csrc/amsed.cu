@@ -252,29 +252,40 @@ int bk_grid(const Handle& h, uint64_t items, uint32_t per_block) {
 }  // namespace
 
 void AmsedPrecond::prepare_block(uint32_t k) {
-    if (bk_ >= k && !blv_.empty()) return;
     cudaStream_t st = h_.stream;
+    // the levels' sweeps for block_columns(k) columns a CTA, on first use
+    const uint32_t cols = block_columns(k, n_), wi = block_width_index(cols);
+    if (blv_.empty() || !(blv_width_ >> wi & 1u)) {
+        if (blv_.empty()) blv_.resize(nlev_);
+        for (uint32_t l = 0; l < nlev_; ++l) {
+            BlockLevel& B = blv_[l];
+            if (a_->fp32) {
+                Sweep<float> lo, up;
+                level_sweeps<float>(*a_->s32, l, lo, up);
+                B.lower[wi].upload_block(lo, h_.info, cols, st);
+                B.upper[wi].upload_block(up, h_.info, cols, st);
+            } else {
+                Sweep<double> lo, up;
+                level_sweeps<double>(*a_->s64, l, lo, up);
+                B.lower[wi].upload_block(lo, h_.info, cols, st);
+                B.upper[wi].upload_block(up, h_.info, cols, st);
+            }
+        }
+        blv_width_ |= 1u << wi;
+    }
+    for (BlockLevel& B : blv_) {
+        B.lower[wi].block_workspace(k, st);
+        B.upper[wi].block_workspace(k, st);
+    }
+    if (bk_ >= k) return;
     tensor_lowrank_ = a_->fp32;
-    const bool first = blv_.empty();
-    if (first) blv_.resize(nlev_);
+    const bool first = bk_ == 0;
     size_t part64 = 1, part32 = 1, t64 = 1, t32 = 1;
     uint32_t max_nfac = 1;
     for (uint32_t l = 0; l < nlev_; ++l) {
         Level& L = lv_[l];
         BlockLevel& B = blv_[l];
         if (first) {
-            // level-order copies of the sweeps (the block sweep kernel's layout)
-            if (a_->fp32) {
-                Sweep<float> lo, up;
-                level_sweeps<float>(*a_->s32, l, lo, up);
-                B.lower.upload(lo, h_.info, LAYOUT_LEVEL, st);
-                B.upper.upload(up, h_.info, LAYOUT_LEVEL, st);
-            } else {
-                Sweep<double> lo, up;
-                level_sweeps<double>(*a_->s64, l, lo, up);
-                B.lower.upload(lo, h_.info, LAYOUT_LEVEL, st);
-                B.upper.upload(up, h_.info, LAYOUT_LEVEL, st);
-            }
             if (L.rank && tensor_lowrank_) {
                 const std::vector<double>& W = a_->fp32 ? a_->s32->levels[l].W : a_->s64->levels[l].W;
                 const std::vector<double>& Hh = a_->fp32 ? a_->s32->levels[l].H : a_->s64->levels[l].H;
@@ -331,11 +342,13 @@ void AmsedPrecond::block_solve_k(cudaStream_t st, int level, uint32_t k, const d
         PRISM_CUDA(cudaMemcpyAsync(out + (size_t)L.nfac * k, in + (size_t)L.nfac * k,
                                    (size_t)(L.nb - L.nfac) * k * sizeof(double), cudaMemcpyDeviceToDevice, st));
     const uint64_t cnt = (uint64_t)L.nfac * k;
-    launch_bt_fill(st, h_, cnt, sweep_tmpk_.get());
-    if (in != out) launch_bt_fill(st, h_, cnt, out);
-    launch_bt_sweep(h_, st, B.lower, k, in, sweep_tmpk_.get());
-    if (in == out) launch_bt_fill(st, h_, cnt, out);
-    launch_bt_sweep(h_, st, B.upper, k, sweep_tmpk_.get(), out);
+    const DevSweep& lo = B.lower[block_width_index(block_columns(k, n_))];
+    const DevSweep& up = B.upper[block_width_index(block_columns(k, n_))];
+    if (!lo.self_filling()) launch_bt_fill(st, h_, cnt, sweep_tmpk_.get());
+    if (in != out && !up.self_filling()) launch_bt_fill(st, h_, cnt, out);
+    launch_bt_sweep(h_, st, lo, k, in, sweep_tmpk_.get());
+    if (in == out && !up.self_filling()) launch_bt_fill(st, h_, cnt, out);
+    launch_bt_sweep(h_, st, up, k, sweep_tmpk_.get(), out);
 }
 
 // x2 += W (H o (W^T xc)) on k columns

@@ -8,9 +8,12 @@
 // exit by a shared-memory tiled transpose.
 //
 // Why a block pays on the sweeps: a triangular sweep is a chain of dependency
-// wavefronts whose latency (two L2 round trips each) does not depend on how
-// many values a row carries.  With k columns one wavefront moves k values per
-// row, so the same chain of latencies serves k solves.
+// wavefronts whose latency hardly depends on how many values a row carries, and a
+// single vector leaves most SMs waiting for it.  The block sweep is the dataflow
+// kernel (flow_sweep.cuh) with 1, 2 or 4 columns a lane: groups of CTAs take the
+// columns, the CTAs of a group the slabs.  (Level order, a warp a row, remains for
+// factors whose slabs do not fit in shared memory; it took 4.2 ms a sweep of IC
+// 192^2 with 64 columns, 0.34 ms now.)
 //
 // Each column follows the recurrence of CG<double>::solve (CG.cpp:34-83) on
 // its own scalars; a column that has converged is frozen (its x and r stop
@@ -442,8 +445,14 @@ void launch_bt_fill(cudaStream_t st, const Handle& h, uint64_t count, double* p)
     PRISM_LAUNCHED();
 }
 
+void launch_flow_block(const Handle& h, cudaStream_t st, const DevSweep& s, uint32_t k, const double* in, double* out);
+
 void launch_bt_sweep(const Handle& h, cudaStream_t st, const DevSweep& s, uint32_t k, const double* in, double* out) {
     if (!s.n) return;
+    if (s.layout == LAYOUT_FLOW) {
+        launch_flow_block(h, st, s, k, in, out);
+        return;
+    }
     if (s.layout != LAYOUT_LEVEL) throw Error(PRISM_ERR_ARG, "block sweep needs the level-order layout");
     void* fn = s.fp32 ? bt_sweep_kernel<float>(s.op) : bt_sweep_kernel<double>(s.op);
     int occ = 0;
@@ -483,29 +492,29 @@ void launch_bt_unpack(cudaStream_t st, const Handle& h, uint32_t n, uint32_t k, 
 }
 
 // ============================================================================
-// Triangular preconditioner on a block (level-order sweeps; the slab layout
-// that the single-vector tuner may have chosen is re-uploaded in level order
-// once, on first use)
+// Triangular preconditioner on a block: copies of the sweeps for block_columns(k)
+// columns a CTA, uploaded on first use
 // ============================================================================
 void TriangularPrecond::apply_batched(cudaStream_t st, uint32_t k, const double* in, double* out) {
     const uint32_t n = h_.A.n;
-    auto level_order = [&](const DevSweep& tuned, DevSweep& mine, bool lower) -> const DevSweep& {
-        if (tuned.layout == LAYOUT_LEVEL) return tuned;
-        if (mine.n != tuned.n) {
-            if (f_->fp32) mine.upload(lower ? f_->lower32 : f_->upper32, h_.info, LAYOUT_LEVEL, h_.stream);
-            else mine.upload(lower ? f_->lower64 : f_->upper64, h_.info, LAYOUT_LEVEL, h_.stream);
-            refresh_level_copy(mine, lower);  // after a device refactorisation: its values
+    const uint32_t cols = block_columns(k, n);
+    auto copy = [&](DevSweep& mine, bool lower) -> const DevSweep& {
+        if (mine.n != n) {
+            if (f_->fp32) mine.upload_block(lower ? f_->lower32 : f_->upper32, h_.info, cols, h_.stream);
+            else mine.upload_block(lower ? f_->lower64 : f_->upper64, h_.info, cols, h_.stream);
+            refresh_block_copy(mine, lower);  // after a device refactorisation: its values
         }
+        mine.block_workspace(k, st);
         return mine;
     };
-    const DevSweep& lo = level_order(lower_, lower_lv_, true);
-    const DevSweep& up = level_order(upper_, upper_lv_, false);
+    const DevSweep& lo = copy(lower_bk_[block_width_index(cols)], true);
+    const DevSweep& up = copy(upper_bk_[block_width_index(cols)], false);
     const size_t nk = (size_t)n * k;
     if (tmpk_.size() < nk) tmpk_.alloc(nk);
-    launch_bt_fill(st, h_, nk, tmpk_.get());
-    if (in != out) launch_bt_fill(st, h_, nk, out);
+    if (!lo.self_filling()) launch_bt_fill(st, h_, nk, tmpk_.get());
+    if (in != out && !up.self_filling()) launch_bt_fill(st, h_, nk, out);
     launch_bt_sweep(h_, st, lo, k, in, tmpk_.get());
-    if (in == out) launch_bt_fill(st, h_, nk, out);
+    if (in == out && !up.self_filling()) launch_bt_fill(st, h_, nk, out);
     launch_bt_sweep(h_, st, up, k, tmpk_.get(), out);
 }
 

@@ -43,7 +43,7 @@ struct SlabPlan {
 
 template <typename Low>
 bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32_t max_slots, FlowLayout& out,
-                 StreamOrder* order, std::vector<uint32_t>* coef_map) {
+                 StreamOrder* order, std::vector<uint32_t>* coef_map, uint32_t entries) {
     const uint32_t n = s.n, ns = (uint32_t)start.size() - 1;
     max_slots = std::min<uint32_t>(max_slots, 0xFFFFu);
     out = FlowLayout();
@@ -51,7 +51,7 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
     const bool recip = s.op == SWEEP_DIV || s.op == SWEEP_PREDIV;
     constexpr uint32_t vb = (uint32_t)sizeof(Low), Q = kFlowLanes;
     // rows of up to 16 positions in one chunk of four a lane
-    const uint32_t E = s.val.size() <= 12 * (uint64_t)n ? 4 : 8, RB = Q * E * (2 + vb);
+    const uint32_t E = entries ? entries : (s.val.size() <= 12 * (uint64_t)n ? 4 : 8), RB = Q * E * (2 + vb);
     out.entries = E;
     auto tail_bytes = [](uint32_t m) { return flow_tail_bytes(m, vb); };
     std::vector<uint32_t> owner(n), slot(n);
@@ -290,9 +290,9 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
     return true;
 }
 template bool flow_layout<double>(const Sweep<double>&, const std::vector<uint32_t>&, uint32_t, FlowLayout&,
-                                  StreamOrder*, std::vector<uint32_t>*);
+                                  StreamOrder*, std::vector<uint32_t>*, uint32_t);
 template bool flow_layout<float>(const Sweep<float>&, const std::vector<uint32_t>&, uint32_t, FlowLayout&,
-                                 StreamOrder*, std::vector<uint32_t>*);
+                                 StreamOrder*, std::vector<uint32_t>*, uint32_t);
 
 namespace {
 template <typename Low, typename Acc>

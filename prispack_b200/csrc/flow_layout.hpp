@@ -63,12 +63,12 @@ struct FlowLayout {
     std::vector<uint32_t> dg_pos;  // per row: its entry of dg
 };
 
-// Lays the sweep out for slabs [start[b], start[b + 1]).  False when a slab needs more
-// than max_slots value slots.  order, coef_map: as for stream_layout (every position is
+// Lays the sweep out for slabs [start[b], start[b + 1]), with E = entries (0: by the rows'
+// lengths).  False when a slab needs more than max_slots value slots.  order, coef_map: as for stream_layout (every position is
 // an early one; coef_map in units of the factor value within `chunks`).
 template <typename Low>
 bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32_t max_slots, FlowLayout& out,
-                 StreamOrder* order = nullptr, std::vector<uint32_t>* coef_map = nullptr);
+                 StreamOrder* order = nullptr, std::vector<uint32_t>* coef_map = nullptr, uint32_t entries = 0);
 
 // Replays k_sweep_flow on the host, in its arithmetic (float when acc32): every index of the
 // layout checked against its array, each worker's tasks taken in order as their values become

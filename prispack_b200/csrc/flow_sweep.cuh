@@ -31,6 +31,10 @@
 //  - There are more slabs than CTAs where a wavefront is wide: a CTA takes its next slab
 //    while the wavefront is elsewhere.
 //
+// Blocks of columns run the same kernel with 1, 2 or 4 columns a lane (block_columns): a record
+// serves them all, groups of CTAs take the columns. Us a sweep, level order before: IC 192^2,
+// 64 columns 4,208, now 311; AMSED 95x71 FP64, 13 columns 485 to 1,540, now 31.
+//
 // Measured against the streamed rounds (us an M^-1 apply): IC 64^2 FP64 150 against 334, IC
 // 512^2 FP64 1,052 against 2,948, ILUT 61x53x47 with float values 388 against 950 (level
 // order), AMSED 64^3 FP64 1,670 against 2,200, AMSED 128^3 with float arithmetic 4,476
@@ -71,7 +75,10 @@ struct FlowArgs {
     double* out;
     int* status;
     unsigned long long wait_ns;
-    uint32_t slabs, slots, members, k;
+    uint32_t slabs, slots;
+    // blocks of columns (interleaved, X[row * k + c]): `members` CTAs a group of columns
+    const double* dd;           // the diagonal itself, per (task, row)
+    uint32_t members, k;
 };
 
 // record words: read once, in order, by one warp
@@ -137,6 +144,15 @@ __device__ __forceinline__ void flow_bar_sync(uint32_t id, uint32_t threads) {
 __device__ __forceinline__ void flow_bar_arrive(uint32_t id, uint32_t threads) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+__device__ __forceinline__ void flow_load2(uint32_t at, double& v, double& w) {
+    asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v), "=d"(w) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void flow_peek2(uint32_t at, double& v, double& w) {
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v), "=d"(w) : "r"(at));
+}
+__device__ __forceinline__ void flow_store2(uint32_t at, double v, double w) {
+    asm volatile("st.volatile.shared.v2.f64 [%0], {%1, %2};" ::"r"(at), "d"(v), "d"(w) : "memory");
+}
 // a first look: may miss a value just written, so only a loop of flow_load may wait
 __device__ __forceinline__ void flow_peek(uint32_t at, float& v) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at));
@@ -151,16 +167,60 @@ __device__ __forceinline__ void flow_store(uint32_t at, double v) {
     asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
 }
 
-template <typename Low, int OP, typename Acc, int E>
+// v / d from r = 1 / d rounded: one step that takes the product's error out again.
+__device__ __forceinline__ double flow_quotient(double v, double d, double r) {
+    const double q = acc_mul(v, r), e = acc_fma(acc_fma(-q, d, v), r, q);
+    return isfinite(q) ? e : q;
+}
+
+// C = 0: one vector.  C = 1, 2, 4: C columns of a block at once (double arithmetic); CTA
+// g * members + m takes the slabs m, m + members, ... for the columns C g .. C g + C - 1.
+template <typename Low, int OP, typename Acc, int E, int C>
 static __global__ void __launch_bounds__(kFlowThreads, 1) k_sweep_flow(const FlowArgs a) {
     extern __shared__ __align__(128) unsigned char fsm[];
-    constexpr uint32_t vb = sizeof(Low), ab = sizeof(Acc);
+    constexpr uint32_t vb = sizeof(Low);
+    constexpr int N = C == 0 ? 1 : C;
     constexpr int CQ = E * (int)vb / 16;         // 16-byte words of a lane's coefficients
     constexpr uint32_t LB = E * (2 + vb);         // bytes of a lane in a chunk
+    constexpr int V = N == 1 ? 1 : 2, PL = N / V; // columns of a slot word, planes of slot words
+    constexpr uint32_t sb = sizeof(Acc) * V;      // bytes of a slot word
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t xs = smem_addr(fsm + kFlowFixedSmem);
+    const uint32_t xs = smem_addr(fsm + kFlowFixedSmem), plane = a.slots * sb;
     volatile uint32_t* leave = reinterpret_cast<volatile uint32_t*>(fsm);
-    FlowWord<Acc>* xch = static_cast<FlowWord<Acc>*>(a.xch);
+    const uint32_t group = C == 0 ? 0u : blockIdx.x / a.members, groups = C == 0 ? 1u : gridDim.x / a.members;
+    const uint32_t first_slab = C == 0 ? blockIdx.x : blockIdx.x % a.members, step = C == 0 ? gridDim.x : a.members;
+    const uint32_t col = group * N;               // first column
+    FlowWord<Acc>* xch = static_cast<FlowWord<Acc>*>(a.xch) + group * N;
+    auto word_of = [&](uint32_t e) { return xch + (C == 0 ? (size_t)e : (size_t)e * (groups * N)); };
+    // the N values of a slot
+    auto peek = [&](uint32_t at, Acc(&x)[N]) {
+        if constexpr (N == 1) {
+            flow_peek(at, x[0]);
+        } else {
+#pragma unroll
+            for (int p = 0; p < PL; ++p) flow_peek2(at + p * plane, x[2 * p], x[2 * p + 1]);
+        }
+    };
+    auto look = [&](uint32_t at, Acc(&x)[N]) {
+        if constexpr (N == 1) {
+            flow_load(at, x[0]);
+        } else {
+#pragma unroll
+            for (int p = 0; p < PL; ++p) flow_load2(at + p * plane, x[2 * p], x[2 * p + 1]);
+        }
+        bool pend = false;
+#pragma unroll
+        for (int j = 0; j < N; ++j) pend = pend || flow_pending(x[j]);
+        return pend;
+    };
+    auto store = [&](uint32_t at, const Acc(&x)[N]) {
+        if constexpr (N == 1) {
+            flow_store(at, x[0]);
+        } else {
+#pragma unroll
+            for (int p = 0; p < PL; ++p) flow_store2(at + p * plane, x[2 * p], x[2 * p + 1]);
+        }
+    };
     uint32_t epoch;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(epoch) : "l"(a.ctl) : "memory");
     ++epoch;
@@ -177,12 +237,15 @@ static __global__ void __launch_bounds__(kFlowThreads, 1) k_sweep_flow(const Flo
             dead = true;
         }
     };
-    for (uint32_t b = blockIdx.x; b < a.slabs; b += gridDim.x) {
+    for (uint32_t b = first_slab; b < a.slabs; b += step) {
         for (uint32_t i = threadIdx.x; i < a.slots; i += blockDim.x) {
             Acc v;
-            if constexpr (ab == 4) v = __uint_as_float(kFlowPendF);
+            if constexpr (sizeof(Acc) == 4) v = __uint_as_float(kFlowPendF);
             else v = __longlong_as_double((long long)kPending);
-            flow_store(xs + i * ab, i == 0 ? (Acc)0 : v);
+            Acc x[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) x[j] = i == 0 ? (Acc)0 : v;
+            store(xs + i * sb, x);
         }
         __syncthreads();
         if (warp < (int)kFlowWorkers) {
@@ -191,18 +254,30 @@ static __global__ void __launch_bounds__(kFlowThreads, 1) k_sweep_flow(const Flo
             const uint32_t nt = wi.z, nch = wi.w;
             const uint4* hp = a.hdr + (size_t)wi.y * kFlowRows + lane / (int)kFlowLanes;
             const Acc* dp = static_cast<const Acc*>(a.dg) + (size_t)wi.y * kFlowRows + lane / (int)kFlowLanes;
+            const double* ep = a.dd + (size_t)wi.y * kFlowRows + lane / (int)kFlowLanes;
             const unsigned char* src = a.chunks + (size_t)we.x * 16;
             for (uint32_t o = (uint32_t)lane * 128; o < kFlowAhead && o < we.y * 16u; o += 4096) prefetch_l2(src + o);
             uint4 h0 = make_uint4(kFlowNone, kFlowNone, 0, 0), h1 = h0;
             Acc d0 = (Acc)1, d1 = (Acc)1;
-            double v0 = 0.0;
+            double e0 = 1.0;
+            double v0[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) v0[j] = 0.0;
             if (nt > 0) h0 = __ldg(hp), d0 = __ldg(dp);
             uint32_t t = 0;
             // the next task's header and this one's right-hand side
             auto ahead = [&]() {
                 h1.x = kFlowNone;
                 if (t + 1 < nt) h1 = __ldg(hp + (size_t)(t + 1) * kFlowRows), d1 = __ldg(dp + (size_t)(t + 1) * kFlowRows);
-                if (h0.x != kFlowNone) v0 = a.in[h0.x];
+                if (C != 0 && (OP == OP_DIV || OP == OP_PREDIV) && t < nt) e0 = __ldg(ep + (size_t)t * kFlowRows);
+                if (h0.x != kFlowNone) {
+                    if constexpr (C == 0) {
+                        v0[0] = a.in[h0.x];
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < N; ++j) v0[j] = col + j < a.k ? a.in[(size_t)h0.x * a.k + col + j] : 0.0;
+                    }
+                }
             };
             ahead();
             // the chunk in work and the next one (lanes without a row read slot 0)
@@ -252,92 +327,116 @@ static __global__ void __launch_bounds__(kFlowThreads, 1) k_sweep_flow(const Flo
                 }
                 src += flow_tail_bytes(m, vb);
             };
-            Acc c = (Acc)0;
+            auto coef_of = [](const uint4& v, int i) {
+                if constexpr (vb == 4)
+                    return (Acc)__uint_as_float((i & 3) == 0 ? v.x : ((i & 3) == 1 ? v.y : ((i & 3) == 2 ? v.z : v.w)));
+                else
+                    return (i & 1) ? __hiloint2double((int)v.w, (int)v.z) : __hiloint2double((int)v.y, (int)v.x);
+            };
+            Acc c[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) c[j] = (Acc)0;
             const bool first = (lane & ((int)kFlowLanes - 1)) == 0;
 #pragma unroll 1
             for (uint32_t ch = 0; ch < nch; ++ch) {
                 if (left == 1) fetch_tail(h0.w >> 8 & 15u);
                 if (ch + 1 < nch) fetch(sn, qn, (left > 1 ? h0.w >> 8 : h0.w >> 12) & 15u);
-                auto at = [&](int i) { return xs + ((sl[i / 2] >> (16 * (i & 1))) & 0xFFFFu) * ab; };
-                auto coef = [&](int i) {
-                    const uint4 v = q[i * (int)vb / 16];
-                    if constexpr (vb == 4)
-                        return (Acc)__uint_as_float((i & 3) == 0 ? v.x : ((i & 3) == 1 ? v.y : ((i & 3) == 2 ? v.z : v.w)));
-                    else
-                        return (i & 1) ? __hiloint2double((int)v.w, (int)v.z) : __hiloint2double((int)v.y, (int)v.x);
-                };
-                // positions [0, n) of the chunk onto c, each value awaited.  A sentinel makes the
-                // chain a NaN: no NaN, nothing was pending.  The warp stays together (lanes that
-                // spin apart starve one another).
-                auto add = [&](int n) {
-                    Acc g = c;
-                    Acc x[E];
+                auto at = [&](int i) { return xs + ((sl[i / 2] >> (16 * (i & 1))) & 0xFFFFu) * sb; };
+                auto coef = [&](int i) { return coef_of(q[i * (int)vb / 16], i); };
+                // the chunk's positions onto c, each value awaited.  A sentinel makes the chain
+                // a NaN: no NaN, nothing was pending.  The warp stays together (lanes that spin
+                // apart starve one another).
+                auto add = [&]() {
+                    constexpr int B = N == 4 ? 4 : E;  // positions in flight
+                    Acc g[N];
 #pragma unroll
-                    for (int i = 0; i < E; ++i)
-                        if (i < n) flow_peek(at(i), x[i]);
+                    for (int j = 0; j < N; ++j) g[j] = c[j];
 #pragma unroll
-                    for (int i = 0; i < E; ++i)
-                        if (i < n) g = acc_fma(coef(i), x[i], g);
-                    if (!__any_sync(0xFFFFFFFFu, g != g)) {
-                        c = g;
+                    for (int i0 = 0; i0 < E; i0 += B) {
+                        Acc x[B][N];
+#pragma unroll
+                        for (int i = 0; i < B; ++i) peek(at(i0 + i), x[i]);
+#pragma unroll
+                        for (int i = 0; i < B; ++i)
+#pragma unroll
+                            for (int j = 0; j < N; ++j) g[j] = acc_fma(coef(i0 + i), x[i][j], g[j]);
+                    }
+                    bool nan = false;
+#pragma unroll
+                    for (int j = 0; j < N; ++j) nan = nan || g[j] != g[j];
+                    if (!__any_sync(0xFFFFFFFFu, nan)) {
+#pragma unroll
+                        for (int j = 0; j < N; ++j) c[j] = g[j];
                         return;
                     }
 #pragma unroll
-                    for (int j = 0; j < E; j += 2) {
-                        if (j < n) {
-                            Acc y[2] = {(Acc)0, (Acc)0};
-                            bool p;
-                            unsigned polls = 0;
-                            do {
-                                flow_load(at(j), y[0]);
-                                if (j + 1 < n) flow_load(at(j + 1), y[1]);
-                                p = __any_sync(0xFFFFFFFFu, flow_pending(y[0]) || flow_pending(y[1])) && !dead;
-                                if (p && ++polls >= kFlowPolls) {
-                                    polls = 0;
-                                    expired();
-                                    dead = __any_sync(0xFFFFFFFFu, dead);
-                                }
-                            } while (p);
-                            c = acc_fma(coef(j), y[0], c);
-                            if (j + 1 < n) c = acc_fma(coef(j + 1), y[1], c);
-                        }
+                    for (int i = 0; i < E; i += 2) {
+                        Acc y[2][N];
+                        bool p;
+                        unsigned polls = 0;
+                        do {
+                            p = look(at(i), y[0]);
+                            p = look(at(i + 1), y[1]) || p;
+                            p = __any_sync(0xFFFFFFFFu, p) && !dead;
+                            if (p && ++polls >= kFlowPolls) {
+                                polls = 0;
+                                expired();
+                                dead = __any_sync(0xFFFFFFFFu, dead);
+                            }
+                        } while (p);
+#pragma unroll
+                        for (int j = 0; j < N; ++j) c[j] = acc_fma(coef(i + 1), y[1][j], acc_fma(coef(i), y[0][j], c[j]));
                     }
                     since = 0;
                 };
-                if (--left != 0) {
-                    add(E);
-                } else {
-                    const Acc vin = (Acc)v0;
-                    const uint32_t slot_at = xs + (h0.z & 0xFFFFu) * ab, sync = h0.w >> 17 & 31u, id = h0.z >> 16 & 15u, arrive = h0.w >> 22;
+                add();
+                if (--left == 0) {
+                    const uint32_t slot_at = xs + (h0.z & 0xFFFFu) * sb, sync = h0.w >> 17 & 31u, id = h0.z >> 16 & 15u, arrive = h0.w >> 22;
                     const bool mine = first && h0.x != kFlowNone;
-                    add(E);
-                    c = acc_add(c, __shfl_xor_sync(0xFFFFFFFFu, c, 1));
-                    Acc s = acc_add(c, __shfl_xor_sync(0xFFFFFFFFu, c, 2));
-                    // the tail: rows of this slab alone, ready once the level before is
-                    Acc res;
-                    if (sync != 0u) flow_bar_sync(id, sync * 32u);
-                    Acc x[4];
+                    Acc s[N], vin[N];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) flow_peek(xs + (((i < 2 ? ts.x : ts.y) >> (16 * (i & 1))) & 0xFFFFu) * ab, x[i]);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        Acc cf;
-                        const uint4 v = tq[i * (int)vb / 16];
-                        if constexpr (vb == 4) cf = (Acc)__uint_as_float(i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)));
-                        else cf = (i & 1) ? __hiloint2double((int)v.w, (int)v.z) : __hiloint2double((int)v.y, (int)v.x);
-                        s = acc_fma(cf, x[i], s);
+                    for (int j = 0; j < N; ++j) {
+                        vin[j] = (Acc)v0[j];
+                        if (OP == OP_PREDIV) {
+                            if constexpr (C == 0) vin[j] = acc_mul(vin[j], d0);
+                            else vin[j] = flow_quotient(vin[j], e0, d0);
+                        }
+                        s[j] = acc_add(c[j], __shfl_xor_sync(0xFFFFFFFFu, c[j], 1));
+                        s[j] = acc_add(s[j], __shfl_xor_sync(0xFFFFFFFFu, s[j], 2));
                     }
-                    if (OP == OP_DIV || OP == OP_MUL) res = acc_mul(acc_sub(vin, s), d0);
-                    else if (OP == OP_NONE) res = acc_sub(vin, s);
-                    else res = acc_sub(acc_mul(vin, d0), s);
-                    if (mine) flow_store(slot_at, res);
+                    // the tail: rows of this slab alone, ready once the level before is
+                    if (sync != 0u) flow_bar_sync(id, sync * 32u);
+                    Acc x[4][N], res[N];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) peek(xs + (((i < 2 ? ts.x : ts.y) >> (16 * (i & 1))) & 0xFFFFu) * sb, x[i]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < N; ++j) s[j] = acc_fma(coef_of(tq[i * (int)vb / 16], i), x[i][j], s[j]);
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        res[j] = acc_sub(vin[j], s[j]);
+                        if (OP == OP_MUL || (OP == OP_DIV && C == 0)) res[j] = acc_mul(res[j], d0);
+                        else if constexpr (OP == OP_DIV && C != 0) res[j] = flow_quotient(res[j], e0, d0);
+                    }
+                    if (mine) store(slot_at, res);
                     if (arrive != 0u) flow_bar_arrive(id == kFlowBars ? 1u : id + 1u, arrive * 32u);
                     if (mine) {
-                        if (h0.y != kFlowNone) FlowWord<Acc>::put(xch + h0.y, res, epoch);
-                        const double rd = (double)res;
-                        a.out[h0.x] = rd != rd ? __longlong_as_double((long long)kCanonicalNaN) : rd;
+                        if (h0.y != kFlowNone) {
+                            FlowWord<Acc>* w = word_of(h0.y);
+#pragma unroll
+                            for (int j = 0; j < N; ++j) FlowWord<Acc>::put(w + j, res[j], epoch);
+                        }
+#pragma unroll
+                        for (int j = 0; j < N; ++j) {
+                            const double rd = (double)res[j];
+                            const double o = rd != rd ? __longlong_as_double((long long)kCanonicalNaN) : rd;
+                            if constexpr (C == 0) a.out[h0.x] = o;
+                            else if (col + j < a.k) a.out[(size_t)h0.x * a.k + col + j] = o;
+                        }
                     }
-                    c = (Acc)0;
+#pragma unroll
+                    for (int j = 0; j < N; ++j) c[j] = (Acc)0;
                     ++t;
                     h0 = h1, d0 = d1;
                     left = h0.w & 0xFFu;
@@ -353,7 +452,7 @@ static __global__ void __launch_bounds__(kFlowThreads, 1) k_sweep_flow(const Flo
             constexpr uint32_t S = 32 * kFlowHaloWarps;
             uint32_t i = __ldg(a.halo_ptr + b) + (uint32_t)(warp - (int)kFlowWorkers) * 32 + (uint32_t)lane;
             // U entries of the list in flight a lane, and the next U known
-            constexpr int U = 4;
+            constexpr int U = N == 1 ? 4 : (N == 2 ? 2 : 1);
             uint2 e[U], nx[U];
             uint32_t at[U];
 #pragma unroll
@@ -365,17 +464,24 @@ static __global__ void __launch_bounds__(kFlowThreads, 1) k_sweep_flow(const Flo
             unsigned idle = 0;
             bool more = true;
             while (__any_sync(0xFFFFFFFFu, more)) {
-                Acc v[U];
+                Acc v[U][N];
                 bool ok[U], some = false;
                 more = false;
-                // no branch between the loads: all U are in flight at once
+                // no branch between the loads: all are in flight at once
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    ok[u] = FlowWord<Acc>::get(xch + (e[u].x != kFlowNone ? e[u].x : 0u), v[u], epoch);
+                for (int u = 0; u < U; ++u) {
+                    const FlowWord<Acc>* w = word_of(e[u].x != kFlowNone ? e[u].x : 0u);
+                    ok[u] = true;
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        const bool in = FlowWord<Acc>::get(w + j, v[u][j], epoch);
+                        ok[u] = in && ok[u];
+                    }
+                }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     if (ok[u] && e[u].x != kFlowNone) {
-                        flow_store(xs + e[u].y * ab, v[u]);
+                        store(xs + e[u].y * sb, v[u]);
                         e[u] = nx[u];
                         nx[u] = at[u] < h1 ? __ldg(a.halo + at[u]) : make_uint2(kFlowNone, 0);
                         at[u] += U * S;

@@ -317,7 +317,7 @@ struct RefactorState {
     DevBuf<double> lt64, D;
     DevBuf<int> status;       // [status, first bad column]
     DevBuf<unsigned> bad;     // first out-of-range map entry: [coefficients, diagonals]
-    SweepValueMap lower, upper, lower_lv, upper_lv;
+    SweepValueMap lower, upper, block;
     bool refactored = false;  // the device factor differs from the host one
 };
 void refactor_release(RefactorState* r) { delete r; }
@@ -342,7 +342,7 @@ void build_map(const DevSweep& d, const Sweep<Low>& s, const Sweep<double>& idx,
     if (d.layout == LAYOUT_FLOW) {
         FlowLayout F;
         std::vector<uint32_t> cmap;
-        if (!flow_layout<Low>(s, slab_ranges<Low>(s, d.str_ctas_req), d.str_slots, F, nullptr, &cmap))
+        if (!flow_layout<Low>(s, slab_ranges<Low>(s, d.str_ctas_req), d.str_slots, F, nullptr, &cmap, d.fl_entries))
             throw Error(PRISM_ERR_CUDA, "dataflow layout could not be rebuilt");
         cd.reserve(cmap.size() / 2);
         cs.reserve(cmap.size() / 2);
@@ -436,6 +436,12 @@ void apply_map(const Handle& h, cudaStream_t st, DevSweep& d, const SweepValueMa
                                                                             D, src_n, ic, recip, dst, dst_n, bad + 1);
         }
         PRISM_LAUNCHED();
+        if (d.fl_cols && recip) {  // blocks hold the diagonals themselves, too
+            k_rf_diag<Low, double><<<rf_grid(h, M.ndiag), kBlock, 0, st>>>(M.ndiag, M.ddst.get(), M.dsrc.get(), lt, D,
+                                                                            src_n, ic, 0, d.fl_dd.get(),
+                                                                            d.fl_dd.size(), bad + 1);
+            PRISM_LAUNCHED();
+        }
     }
 }
 }  // namespace
@@ -596,22 +602,22 @@ void TriangularPrecond::refactor() {
         apply_map<double>(h_, st, upper_, R.upper, R.lt64.get(), lt_n, D, ic, R.bad.get());
     }
     check_maps(R, st, "the sweeps");
-    // the level-order copies of the block solves are uploaded again on their next use, with
-    // the new values (refresh_level_copy)
-    lower_lv_.release();
-    upper_lv_.release();
+    // the copies of the block solves are uploaded again on their next use, with the new
+    // values (refresh_block_copy)
+    for (DevSweep& d : lower_bk_) d.release();
+    for (DevSweep& d : upper_bk_) d.release();
     R.refactored = true;
     PRISM_CUDA(cudaStreamSynchronize(st));
 }
 
-void TriangularPrecond::refresh_level_copy(DevSweep& d, bool lower) {
+void TriangularPrecond::refresh_block_copy(DevSweep& d, bool lower) {
     if (!rf_ || !rf_->refactored) return;
     const HostFactor& F = *f_;
     RefactorState& R = *rf_;
     cudaStream_t st = h_.stream;
     Sweep<double> ilo, iup;
     factor_index_sweeps(F, ilo, iup);
-    SweepValueMap& M = lower ? R.lower_lv : R.upper_lv;
+    SweepValueMap& M = R.block;
     const uint64_t lt_n = F.f0.col.size();
     PRISM_CUDA(cudaMemsetAsync(R.bad.get(), 0, 2 * sizeof(unsigned), st));
     if (F.fp32) {
@@ -621,7 +627,7 @@ void TriangularPrecond::refresh_level_copy(DevSweep& d, bool lower) {
         build_map<double>(d, lower ? F.lower64 : F.upper64, lower ? ilo : iup, M, st);
         apply_map<double>(h_, st, d, M, R.lt64.get(), lt_n, R.D.get(), F.kind == 1, R.bad.get());
     }
-    check_maps(R, st, "a level-order copy");
+    check_maps(R, st, "a block copy");
 }
 
 int TriangularPrecond::export_refactored(int which, uint32_t* n, uint64_t* nnz, uint32_t* rowptr, uint32_t* col,

@@ -30,6 +30,10 @@ constexpr int kSpmvG = 1, kSpmvU = 2;                  // k_spmv: lanes per row,
 // IC 512^2 FP64 1590 / 1269 / 1052, IC 40^3 FP64 437 / 473 / 580, AMSED 128^3 with float
 // arithmetic 4971 / 4476 / 5649.
 constexpr uint32_t kFlowSlabRows[3] = {1024, 2048, 4096};
+// Rows of a slab of a block sweep: as many slabs as let the few CTAs of a group keep up with the
+// wavefront (512^2, k = 64, 2 columns: 5,266 us with 2,048 rows, 3,047 with 4,096; 192^2: 682 with
+// 1,024, 805 with 2,048).
+static uint32_t block_slab_rows(uint32_t n) { return std::max(1024u, n / 64u); }
 constexpr int kSpmvShapes = 6;
 constexpr int kSpmvShapeG[kSpmvShapes] = {1, 1, 2, 4, 8, 16};
 constexpr int kSpmvShapeU[kSpmvShapes] = {2, 4, 2, 1, 1, 1};
@@ -93,23 +97,69 @@ static void* stream_kernel(bool fp32, int op, bool acc32) {
     }
 }
 
-// acc32 as above; entries: E of the layout
-template <typename Low, typename Acc, int E>
+// acc32 as above; entries: E of the layout; cols: as DevSweep::fl_cols (4 entries where not 0)
+template <typename Low, typename Acc, int E, int C>
 static void* flow_kernel_of(int op) {
     switch (op) {
-        case SWEEP_DIV: return (void*)k_sweep_flow<Low, OP_DIV, Acc, E>;
-        case SWEEP_MUL: return (void*)k_sweep_flow<Low, OP_MUL, Acc, E>;
-        case SWEEP_NONE: return (void*)k_sweep_flow<Low, OP_NONE, Acc, E>;
-        default: return (void*)k_sweep_flow<Low, OP_PREDIV, Acc, E>;
+        case SWEEP_DIV: return (void*)k_sweep_flow<Low, OP_DIV, Acc, E, C>;
+        case SWEEP_MUL: return (void*)k_sweep_flow<Low, OP_MUL, Acc, E, C>;
+        case SWEEP_NONE: return (void*)k_sweep_flow<Low, OP_NONE, Acc, E, C>;
+        default: return (void*)k_sweep_flow<Low, OP_PREDIV, Acc, E, C>;
     }
 }
-static void* flow_kernel(bool fp32, int op, bool acc32, uint32_t entries) {
-    if (entries == 4) {
-        if (acc32) return flow_kernel_of<float, float, 4>(op);
-        return fp32 ? flow_kernel_of<float, double, 4>(op) : flow_kernel_of<double, double, 4>(op);
+static void* flow_kernel(bool fp32, int op, bool acc32, uint32_t entries, uint32_t cols) {
+    switch (cols) {
+        case 1: return fp32 ? flow_kernel_of<float, double, 4, 1>(op) : flow_kernel_of<double, double, 4, 1>(op);
+        case 2: return fp32 ? flow_kernel_of<float, double, 4, 2>(op) : flow_kernel_of<double, double, 4, 2>(op);
+        case 4: return fp32 ? flow_kernel_of<float, double, 4, 4>(op) : flow_kernel_of<double, double, 4, 4>(op);
+        default: break;
     }
-    if (acc32) return flow_kernel_of<float, float, 8>(op);
-    return fp32 ? flow_kernel_of<float, double, 8>(op) : flow_kernel_of<double, double, 8>(op);
+    if (entries == 4) {
+        if (acc32) return flow_kernel_of<float, float, 4, 0>(op);
+        return fp32 ? flow_kernel_of<float, double, 4, 0>(op) : flow_kernel_of<double, double, 4, 0>(op);
+    }
+    if (acc32) return flow_kernel_of<float, float, 8, 0>(op);
+    return fp32 ? flow_kernel_of<float, double, 8, 0>(op) : flow_kernel_of<double, double, 8, 0>(op);
+}
+
+static FlowArgs flow_args(const Handle& h, const DevSweep& s, const double* in, double* out) {
+    FlowArgs a;
+    a.chunks = s.fl_chunks.get();
+    a.hdr = reinterpret_cast<const uint4*>(s.fl_hdr.get());
+    a.dg = s.fl_dg.get();
+    a.warp = reinterpret_cast<const uint4*>(s.fl_warp.get());
+    a.halo_ptr = s.fl_halo_ptr.get();
+    a.halo = reinterpret_cast<const uint2*>(s.fl_halo.get());
+    a.xch = s.fl_xch.get();
+    a.ctl = s.fl_ctl.get();
+    a.in = in;
+    a.out = out;
+    a.status = h.status.get();
+    a.wait_ns = kWaitNs;
+    a.slabs = s.fl_slabs;
+    a.slots = s.str_slots;
+    a.dd = s.fl_dd.get();
+    a.members = s.str_ctas;
+    a.k = 1;
+    return a;
+}
+
+// Columns a CTA of a block sweep takes, for k columns of an n-row operator.  One column has
+// the shortest chain as long as the groups of CTAs that share the slabs are six or more; wider
+// ones read a record for more columns.  Measured (us an IC apply, float values; 1 / 2 / 4
+// columns): 192^2, k = 24: 524 / 560 / 764; 192^2, k = 64: 909 / 682 / 836; 512^2, k = 64:
+// - / 3,047 / 2,672.
+uint32_t block_columns(uint32_t k, uint32_t n) { return k <= 24 ? 1u : (n < 131072 ? 2u : 4u); }
+
+void launch_flow_block(const Handle& h, cudaStream_t st, const DevSweep& s, uint32_t k, const double* in, double* out) {
+    FlowArgs a = flow_args(h, s, in, out);
+    const uint32_t groups = (k + s.fl_cols - 1) / s.fl_cols;
+    a.members = std::max(1u, std::min((uint32_t)h.info.sms / groups, s.fl_slabs));
+    a.k = k;
+    void* args[] = {&a};
+    PRISM_CUDA(cudaLaunchCooperativeKernel(flow_kernel(s.fp32, s.op, false, s.fl_entries, s.fl_cols),
+                                           dim3(groups * a.members), dim3(kFlowThreads), args, s.str_smem, st));
+    PRISM_LAUNCHED();
 }
 
 void launch_sweep_prepare(const Handle& h, cudaStream_t st, const DevSweep& s, const double* in, double* out) {
@@ -155,23 +205,9 @@ void launch_sweep_prepare(const Handle& h, cudaStream_t st, const DevSweep& s, c
 void launch_sweep_kernel(const Handle& h, cudaStream_t st, const DevSweep& s, const double* in, double* out) {
     if (!s.n) return;
     if (s.layout == LAYOUT_FLOW) {
-        FlowArgs a;
-        a.chunks = s.fl_chunks.get();
-        a.hdr = reinterpret_cast<const uint4*>(s.fl_hdr.get());
-        a.dg = s.fl_dg.get();
-        a.warp = reinterpret_cast<const uint4*>(s.fl_warp.get());
-        a.halo_ptr = s.fl_halo_ptr.get();
-        a.halo = reinterpret_cast<const uint2*>(s.fl_halo.get());
-        a.xch = s.fl_xch.get();
-        a.ctl = s.fl_ctl.get();
-        a.in = s.paired ? s.pair_rhs.get() : in;
-        a.out = out;
-        a.status = h.status.get();
-        a.wait_ns = kWaitNs;
-        a.slabs = s.fl_slabs;
-        a.slots = s.str_slots;
+        FlowArgs a = flow_args(h, s, s.paired ? s.pair_rhs.get() : in, out);
         void* args[] = {&a};
-        PRISM_CUDA(cudaLaunchCooperativeKernel(flow_kernel(s.fp32, s.op, s.acc32, s.fl_entries), dim3(s.str_ctas), dim3(kFlowThreads),
+        PRISM_CUDA(cudaLaunchCooperativeKernel(flow_kernel(s.fp32, s.op, s.acc32, s.fl_entries, 0), dim3(s.str_ctas), dim3(kFlowThreads),
                                                args, s.str_smem, st));
         PRISM_LAUNCHED();
         return;
@@ -366,12 +402,15 @@ void init_device_info(DeviceInfo& info, int device) {
             PRISM_CUDA(cudaFuncSetAttribute(stream_kernel(f32, op, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             info.max_smem_optin));
             for (uint32_t e : {4u, 8u}) {
-                PRISM_CUDA(cudaFuncSetAttribute(flow_kernel(f32, op, false, e), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                info.max_smem_optin));
+                PRISM_CUDA(cudaFuncSetAttribute(flow_kernel(f32, op, false, e, 0),
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, info.max_smem_optin));
                 if (f32)
-                    PRISM_CUDA(cudaFuncSetAttribute(flow_kernel(true, op, true, e),
+                    PRISM_CUDA(cudaFuncSetAttribute(flow_kernel(true, op, true, e, 0),
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, info.max_smem_optin));
             }
+            for (uint32_t c : {1u, 2u, 4u})
+                PRISM_CUDA(cudaFuncSetAttribute(flow_kernel(f32, op, false, 4, c),
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, info.max_smem_optin));
             if (f32)
                 PRISM_CUDA(cudaFuncSetAttribute(stream_kernel(true, op, true),
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, info.max_smem_optin));
@@ -488,7 +527,8 @@ void DevSweep::release() {
     str_round_cap = 0;
     fl_chunks.release(); fl_dg.release(); fl_xch.release();
     fl_hdr.release(); fl_warp.release(); fl_halo_ptr.release(); fl_halo.release(); fl_ctl.release();
-    fl_slabs = 0;
+    fl_slabs = fl_entries = fl_published = fl_cols = 0;
+    fl_dd.release();
     pair_ptr.release(); pair_dep.release(); pair_coef.release(); pair_rhs.release();
     paired = false;
     n = num_levels = 0;  // empty: nothing launches on a released sweep
@@ -555,7 +595,8 @@ template StreamPlan plan_stream<double>(const Sweep<double>&, const DeviceInfo&,
 template StreamPlan plan_stream<float>(const Sweep<float>&, const DeviceInfo&, bool, bool);
 
 template <typename Low>
-StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows) {
+StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows,
+                     uint32_t cols) {
     StreamPlan P;
     const uint32_t nn = sweep.n;
     if (nn == 0) return P;
@@ -563,13 +604,14 @@ StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32
     if (pair) pair_sweep<Low>(sweep, ps, P.pm);
     const Sweep<Low>& s0 = pair ? ps : sweep;
     P.a32 = acc32 && std::is_same<Low, float>::value;
-    P.slot_bytes = P.a32 ? 4 : 8;
+    P.cols = cols;
+    P.slot_bytes = (P.a32 ? 4 : 8) * std::max(cols, 1u);
     const uint32_t cap = ((uint32_t)info.max_smem_optin - flow_smem(0, P.slot_bytes)) / P.slot_bytes;
     // A slab whose rows and halo do not fit in shared memory is split further.
     uint32_t want = std::max(1u, (nn + rows - 1) / rows);
     for (;; want *= 2) {
         const std::vector<uint32_t> start = slab_ranges<Low>(s0, want);
-        if (flow_layout<Low>(s0, start, cap, P.F)) break;
+        if (flow_layout<Low>(s0, start, cap, P.F, nullptr, nullptr, cols ? 4 : 0)) break;
         if (nn / want < 64) return P;
     }
     P.ok = P.flow = true;
@@ -584,8 +626,8 @@ StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32
     P.nnz = s0.val.size();
     return P;
 }
-template StreamPlan plan_flow<double>(const Sweep<double>&, const DeviceInfo&, bool, bool, uint32_t);
-template StreamPlan plan_flow<float>(const Sweep<float>&, const DeviceInfo&, bool, bool, uint32_t);
+template StreamPlan plan_flow<double>(const Sweep<double>&, const DeviceInfo&, bool, bool, uint32_t, uint32_t);
+template StreamPlan plan_flow<float>(const Sweep<float>&, const DeviceInfo&, bool, bool, uint32_t, uint32_t);
 
 void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
     const StreamLayout& L = P.L;
@@ -627,9 +669,19 @@ void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
         } else {
             fl_dg.upload(reinterpret_cast<const unsigned char*>(F.dg.data()), F.dg.size() * sizeof(double), st);
         }
-        // epoch 0 everywhere: the first sweep is epoch 1
-        fl_xch.alloc((size_t)std::max(F.published, 1u) * (acc32 ? sizeof(FlowWord<float>) : sizeof(FlowWord<double>)));
-        PRISM_CUDA(cudaMemsetAsync(fl_xch.get(), 0, fl_xch.size(), st));
+        fl_cols = P.cols;
+        fl_published = F.published;
+        if (fl_cols) {
+            std::vector<double> dd(F.dg.size(), 1.0);
+            if (op == SWEEP_DIV || op == SWEEP_PREDIV)
+                for (uint32_t r = 0; r < n; ++r) dd[F.dg_pos[r]] = P.diag[r];
+            fl_dd.upload(dd.data(), dd.size(), st);
+            PRISM_CUDA(cudaStreamSynchronize(st));
+        } else {
+            // epoch 0 everywhere: the first sweep is epoch 1
+            fl_xch.alloc((size_t)std::max(F.published, 1u) * (acc32 ? sizeof(FlowWord<float>) : sizeof(FlowWord<double>)));
+            PRISM_CUDA(cudaMemsetAsync(fl_xch.get(), 0, fl_xch.size(), st));
+        }
         fl_ctl.alloc(2);
         PRISM_CUDA(cudaMemsetAsync(fl_ctl.get(), 0, 2 * sizeof(uint32_t), st));
         if (paired) pair_rhs.alloc(n);
@@ -654,6 +706,34 @@ void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
     if (str_halo_row.size() == 0) str_halo_row.alloc(1);  // valid pointers for the kernel
     if (str_halo_sw.size() == 0) str_halo_sw.alloc(1);
     PRISM_CUDA(cudaStreamSynchronize(st));
+}
+
+template <typename Low>
+void DevSweep::upload_block(const Sweep<Low>& s, const DeviceInfo& info, uint32_t cols, cudaStream_t st) {
+    if (s.n > 0) {
+        StreamPlan P = plan_flow<Low>(s, info, false, false, info.flow_rows ? info.flow_rows : block_slab_rows(s.n),
+                                         cols);
+        if (P.ok) {
+            if (s.op == SWEEP_DIV || s.op == SWEEP_PREDIV) {
+                P.diag.resize(s.n);
+                for (uint32_t p = 0; p < s.n; ++p) P.diag[s.order[p]] = s.diag[p];
+            }
+            commit_stream(std::move(P), st);
+            return;
+        }
+    }
+    upload(s, info, LAYOUT_LEVEL, st);
+}
+template void DevSweep::upload_block<double>(const Sweep<double>&, const DeviceInfo&, uint32_t, cudaStream_t);
+template void DevSweep::upload_block<float>(const Sweep<float>&, const DeviceInfo&, uint32_t, cudaStream_t);
+
+void DevSweep::block_workspace(uint32_t k, cudaStream_t st) {
+    if (!fl_cols) return;
+    const size_t groups = (k + fl_cols - 1) / fl_cols;
+    const size_t bytes = std::max(fl_published, 1u) * groups * fl_cols * sizeof(FlowWord<double>);
+    if (fl_xch.size() >= bytes) return;
+    fl_xch.alloc(bytes);
+    PRISM_CUDA(cudaMemsetAsync(fl_xch.get(), 0, bytes, st));  // no entry of the epochs to come
 }
 
 template <typename Low>

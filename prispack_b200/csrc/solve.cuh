@@ -67,6 +67,8 @@ enum SweepLayout : int { LAYOUT_LEVEL = 0, LAYOUT_SLAB = 1, LAYOUT_STREAM = 2, L
 // ok false: the sweep does not fit.
 struct StreamPlan {
     bool ok = false, paired = false, fp32 = false, a32 = false, flow = false;
+    uint32_t cols = 0;             // of a block, per CTA (0: single vectors)
+    std::vector<double> diag;      // blocks of dividing sweeps: the diagonal, by row
     StreamLayout L;
     FlowLayout F;
     PairMap pm;
@@ -79,7 +81,12 @@ template <typename Low>
 StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair);
 // rows: of a slab (fewer where a slab's rows and halo do not fit in shared memory)
 template <typename Low>
-StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows);
+StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows,
+                     uint32_t cols = 0);
+// the columns a CTA takes of a block of k, n rows
+uint32_t block_columns(uint32_t k, uint32_t n);
+constexpr uint32_t kBlockWidths = 3;  // 1, 2 or 4 columns a CTA
+inline uint32_t block_width_index(uint32_t cols) { return cols == 4 ? 2u : cols - 1u; }
 
 struct DevSweep {
     uint32_t n = 0, num_levels = 0;
@@ -102,8 +109,10 @@ struct DevSweep {
     uint32_t str_round_cap = 0;                     // ... and its record cap (0: none)
     // LAYOUT_FLOW (k_sweep_flow): see FlowLayout; str_ctas_req slabs, str_slots, str_smem and
     // str_nnz as above
-    uint32_t fl_slabs = 0, fl_entries = 0;
+    uint32_t fl_slabs = 0, fl_entries = 0, fl_published = 0;
+    uint32_t fl_cols = 0;          // columns a CTA takes of a block (0: single vectors)
     DevBuf<unsigned char> fl_chunks, fl_dg, fl_xch;
+    DevBuf<double> fl_dd;          // blocks: the diagonals beside their reciprocals
     DevBuf<uint32_t> fl_hdr, fl_warp, fl_halo_ptr, fl_halo, fl_ctl;
     // LAYOUT_STREAM or LAYOUT_FLOW built from the paired sweep (pair_sweep): the right-hand side
     // map the prep applies before the kernel (LAYOUT_FLOW: into pair_rhs)
@@ -116,6 +125,11 @@ struct DevSweep {
     template <typename Low>
     bool upload(const Sweep<Low>& s, const DeviceInfo& info, int layout, cudaStream_t st, bool pair = false);
     void commit_stream(StreamPlan&& plan, cudaStream_t st);
+    // Uploads the sweep for blocks of columns, `cols` of them a CTA (block_columns): dataflow
+    // slabs, level order where they do not fit.
+    template <typename Low>
+    void upload_block(const Sweep<Low>& s, const DeviceInfo& info, uint32_t cols, cudaStream_t st);
+    void block_workspace(uint32_t k, cudaStream_t st);  // exchange entries for k columns
     bool streamed() const { return layout == LAYOUT_STREAM || layout == LAYOUT_FLOW; }
     // the streamed layouts mark their own output pending or need no mark; the others need launch_fill first
     bool self_filling() const { return streamed(); }
@@ -198,11 +212,11 @@ class TriangularPrecond : public Precond {
   private:
     int export_refactored(int which, uint32_t* n, uint64_t* nnz, uint32_t* rowptr, uint32_t* col, double* val,
                           double* diag) const;
-    void refresh_level_copy(DevSweep& d, bool lower);
+    void refresh_block_copy(DevSweep& d, bool lower);
     Handle& h_;
     std::shared_ptr<const HostFactor> f_;
     DevSweep lower_, upper_;
-    DevSweep lower_lv_, upper_lv_;   // level-order copies for the block sweeps when the tuner chose slabs
+    DevSweep lower_bk_[kBlockWidths], upper_bk_[kBlockWidths];  // copies for the block sweeps, by block_columns
     DevBuf<double> tmp_, tmpk_;
     std::unique_ptr<RefactorState, void (*)(RefactorState*)> rf_{nullptr, refactor_release};
 };
@@ -254,7 +268,7 @@ class AmsedPrecond : public Precond {
     void c_solve(cudaStream_t st, int level, double* x);
     // block apply (built on first use for a given k)
     struct BlockLevel {
-        DevSweep lower, upper;            // level-order copies of the level's sweeps
+        DevSweep lower[kBlockWidths], upper[kBlockWidths];  // the level's sweeps for blocks, by block_columns
         uint32_t rpad = 0, ldw = 0;       // rank rounded up to 16, rows rounded up to 16
         DevBuf<uint16_t> Wc, Wr;          // BF16 W: column-major rpad x ldw, row-major ldw x rpad
         DevBuf<float> H32;                // [rpad], zero padded
@@ -265,6 +279,7 @@ class AmsedPrecond : public Precond {
     void c_solve_k(cudaStream_t st, int level, uint32_t k, double* x);
     void lowrank_k(cudaStream_t st, int level, uint32_t k, const double* xc, double* y);
     std::vector<BlockLevel> blv_;
+    uint32_t blv_width_ = 0;              // block widths the levels' sweeps are uploaded for, as bits
     uint32_t bk_ = 0;                     // columns the block workspace holds
     bool tensor_lowrank_ = false;         // BF16 tensor-core low-rank products (FP32 factor values)
     DevBuf<double> Xk_, sweep_tmpk_, lr_t64_, lr_part64_;

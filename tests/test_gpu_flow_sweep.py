@@ -69,3 +69,27 @@ def test_random_patterns(env, kind):
     S = P.DeviceSystem(P.CSRMatrix(A.indptr, A.indices, A.data))
     S.set_precond(kind, tol=1e-6, lfill=60)
     check(S, False)
+
+
+@pytest.mark.parametrize("grid,ks,precision", [
+    ((1, 1, 1), (1, 64), P.PRISM_FP64), ((9, 1, 1), (2, 25), P.PRISM_FP64),        # smaller than a task, a chain
+    ((40, 33, 1), (1, 2, 3, 24, 25, 63, 64), P.PRISM_FP32),                        # both sides of each width's limits
+    ((14, 13, 12), (1, 13, 27, 64), P.PRISM_FP64),                                 # rows of several chunks
+    ((364, 361, 1), (25, 63), P.PRISM_FP32)])                                      # four columns a lane
+@pytest.mark.parametrize("kind", [P.PRECOND_IC, P.PRECOND_ILDLT])
+def test_block_columns(grid, ks, precision, kind):
+    """Each column of a block against the single-vector apply: the same factor values in double
+    arithmetic, summed in another order (rows of up to 30 entries, all within 1e-12)."""
+    import torch
+    A = P.CSRMatrix.laplacian(*grid)
+    S = P.DeviceSystem(A)
+    S.set_stream(torch.cuda.current_stream().cuda_stream)
+    S.set_precond(kind, tol=1e-3, precision=precision)
+    for k in ks:
+        g = torch.Generator(device="cuda").manual_seed(k)
+        V = torch.randn(k, A.n, generator=g, device="cuda", dtype=torch.float64)
+        for _ in range(2):
+            out = S.apply_batched(V)
+        for c in {0, k // 2, k - 1}:
+            one = S.apply(V[c].contiguous())
+            assert float((out[c] - one).abs().max()) <= 1e-12 * float(one.abs().max()), (k, c)

@@ -249,6 +249,8 @@ int bk_grid(const Handle& h, uint64_t items, uint32_t per_block) {
     if (want < 1) want = 1;
     return (int)(want < cap ? want : cap);
 }
+// blocks of k_lr_dots_f64
+int lr_grid(int sms, uint32_t nrem) { return (int)std::max(1u, std::min((nrem + kLrTile - 1) / kLrTile, (uint32_t)sms)); }
 }  // namespace
 
 void AmsedPrecond::prepare_block(uint32_t k) {
@@ -311,7 +313,7 @@ void AmsedPrecond::prepare_block(uint32_t k) {
             B.tmp.alloc(std::max<size_t>((size_t)L.nb * k, 1));
             B.tmp2.alloc(std::max<size_t>((size_t)L.nb * k, 1));
             if (L.rank) {
-                part64 = std::max(part64, (size_t)bk_grid(h_, L.nrem, 64) * L.rank * kLrMaxK);
+                part64 = std::max(part64, (size_t)lr_grid(h_.info.sms, L.nrem) * L.rank * kLrMaxK);
                 t64 = std::max(t64, (size_t)L.rank * kLrMaxK);
                 if (tensor_lowrank_) {
                     part32 = std::max(part32, (size_t)bk_grid(h_, B.ldw / 16, kBlock / 32) * B.rpad * kLrMaxK);
@@ -365,7 +367,7 @@ void AmsedPrecond::lowrank_k(cudaStream_t st, int level, uint32_t k, const doubl
                                              lr_t32_.get(), y);
         PRISM_LAUNCHED();
     } else {
-        const int g = bk_grid(h_, L.nrem, 64);
+        const int g = lr_grid(h_.info.sms, L.nrem);
         k_lr_dots_f64<<<g, kBlock, 0, st>>>(L.nrem, k, L.rank, L.W.get(), L.H.get(), xc, lr_part64_.get(),
                                             lr_ticket_.get(), lr_t64_.get());
         PRISM_LAUNCHED();
@@ -469,7 +471,7 @@ void lowrank_block_run(int device, uint32_t nrem, uint32_t rank, uint32_t k, con
         DevBuf<double> dW, dH, dT((size_t)rank * kLrMaxK);
         dW.upload(W, (size_t)rank * nrem, st);
         dH.upload(H, rank, st);
-        const int g = grid(nrem, 64);
+        const int g = lr_grid(info.sms, nrem);
         DevBuf<double> part((size_t)g * rank * kLrMaxK);
         k_lr_dots_f64<<<g, kBlock, 0, st>>>(nrem, k, rank, dW.get(), dH.get(), dX.get(), part.get(), ticket.get(),
                                             dT.get());

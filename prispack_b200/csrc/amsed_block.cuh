@@ -100,6 +100,9 @@ static __global__ void __launch_bounds__(kBlock) k_bk_sub(uint64_t count, const 
 // Block partials of W^T X for rank columns q and block columns c: thread (g, c) with
 // g = threadIdx.x / 64 sums q = g, g + 4, ... over the block's rows (grid-stride by
 // blocks of 64 rows); the last block adds the partials in block order and scales by H.
+// Rows a block takes at a time, and at most one block an SM: with 64 rows a block, six blocks
+// worked on the 371 rows below the first level of a 95 x 71 grid (13 columns: 33 us).
+constexpr uint32_t kLrTile = 8;
 static __global__ void __launch_bounds__(kBlock) k_lr_dots_f64(uint32_t nrem, uint32_t k, uint32_t r,
                                                                const double* __restrict__ W, const double* __restrict__ H,
                                                                const double* __restrict__ X, double* __restrict__ partial,
@@ -110,8 +113,9 @@ static __global__ void __launch_bounds__(kBlock) k_lr_dots_f64(uint32_t nrem, ui
 #pragma unroll
         for (int t = 0; t < 8; ++t) acc[t] = 0.0;
         if (c < k) {
-            for (uint32_t i0 = blockIdx.x * 64; i0 < nrem; i0 += gridDim.x * 64) {
-                const uint32_t i1 = min(nrem, i0 + 64);
+            for (uint32_t i0 = blockIdx.x * kLrTile; i0 < nrem; i0 += gridDim.x * kLrTile) {
+                const uint32_t i1 = min(nrem, i0 + kLrTile);
+#pragma unroll 4
                 for (uint32_t i = i0; i < i1; ++i) {
                     const double x = X[(uint64_t)i * k + c];
 #pragma unroll
@@ -141,6 +145,7 @@ static __global__ void __launch_bounds__(kBlock) k_lr_dots_f64(uint32_t nrem, ui
         const uint32_t q = e / kLrMaxK, cc = e % kLrMaxK;
         if (cc >= k) continue;
         double s = 0.0;
+#pragma unroll 4
         for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(partial + ((size_t)b * r + q) * kLrMaxK + cc);
         T[(size_t)q * kLrMaxK + cc] = s * H[q];
     }

@@ -21,6 +21,7 @@
 // column ends with the iterate, iteration count and error the single solve
 // would report.  Reductions are per column and deterministic (fixed-order
 // block and grid sums).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -34,6 +35,10 @@ namespace {
 
 constexpr int kBK = 64;                                 // columns per block solve
 constexpr int kBWarps = kBlock / 32;                    // warps per block
+// Block size of the kernels that reduce: one block an SM, so that the last block has 148 partial
+// rows to add up rather than 592, each thread a few of them (n = 6,745, 13 columns, us a kernel:
+// 24 with four blocks an SM and one thread a column over all partials).
+constexpr int kRBlock = 1024, kRWarps = kRBlock / 32;
 constexpr unsigned long long kBWaitNs = 1000000000ull;  // 1 s per dependency wait
 
 // Scalar slots of the batched reductions, each kBK wide.
@@ -49,8 +54,9 @@ struct BSlot {
 // partial sum for column lane + 32 h.  Same grid => same bits.
 template <int NV>
 __device__ __forceinline__ void bt_reduce(double (&v)[NV][2], BSlot slot) {
-    static_assert(NV * kBK <= kBlock, "one thread per (value, column)");
-    __shared__ double sm[kBWarps][NV][kBK];
+    constexpr int kCols = NV * kBK, kParts = kRBlock / kCols;  // threads a column when adding up
+    static_assert(kRBlock % kCols == 0, "whole parts");
+    __shared__ double sm[kRWarps][NV][kBK];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
@@ -59,27 +65,38 @@ __device__ __forceinline__ void bt_reduce(double (&v)[NV][2], BSlot slot) {
         sm[wid][q][lane + 32] = v[q][1];
     }
     __syncthreads();
-    const int t = threadIdx.x;
-    if (t < NV * kBK) {
-        const int q = t / kBK, c = t % kBK;
-        double s = 0.0;
+    const int t = threadIdx.x % kCols, part = threadIdx.x / kCols;
+    const int q = t / kBK, c = t % kBK;
+    // the block's warps, then the blocks: each part a share in order, the parts in order
+    auto add_parts = [&](double s) {
+        __syncthreads();
+        sm[part][q][c] = s;
+        __syncthreads();
+        s = 0.0;
+        if (part == 0)
 #pragma unroll
-        for (int w = 0; w < kBWarps; ++w) s += sm[w][q][c];
+            for (int w = 0; w < kParts; ++w) s += sm[w][q][c];
+        return s;
+    };
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < kRWarps / kParts; ++w) s += sm[part * (kRWarps / kParts) + w][q][c];
+    s = add_parts(s);
+    if (part == 0) {
         slot.partial[((size_t)blockIdx.x * NV + q) * kBK + c] = s;
         __threadfence();
     }
     __syncthreads();
-    if (t == 0) last = atomicAdd(slot.ticket, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) last = atomicAdd(slot.ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (t < NV * kBK) {
-        const int q = t / kBK, c = t % kBK;
-        double s = 0.0;
-        for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(slot.partial + ((size_t)b * NV + q) * kBK + c);
-        slot.out[q * kBK + c] = s;
-    }
-    if (t == 0) *slot.ticket = 0u;
+    s = 0.0;
+#pragma unroll 4
+    for (unsigned b = part; b < gridDim.x; b += kParts) s += __ldcg(slot.partial + ((size_t)b * NV + q) * kBK + c);
+    s = add_parts(s);
+    if (part == 0) slot.out[q * kBK + c] = s;
+    if (threadIdx.x == 0) *slot.ticket = 0u;
 }
 
 // column-major (ld) <-> interleaved, 32 rows x k columns per block through shared memory
@@ -124,7 +141,7 @@ __global__ void __launch_bounds__(kBlock) k_bt_unpack(uint32_t n, uint32_t k, ui
 
 // Y = A X (interleaved, warp per row); NDOT = 1: Σ y z per column; NDOT = 2: also Σ x q.
 template <int NDOT>
-__global__ void __launch_bounds__(kBlock) k_bt_spmm(uint32_t n, uint32_t k, const uint32_t* __restrict__ rowptr,
+__global__ void __launch_bounds__(NDOT > 0 ? kRBlock : kBlock) k_bt_spmm(uint32_t n, uint32_t k, const uint32_t* __restrict__ rowptr,
                                                     const uint32_t* __restrict__ col, const double* __restrict__ val,
                                                     const double* __restrict__ X, double* __restrict__ Y,
                                                     const double* __restrict__ Z, const double* __restrict__ Q,
@@ -168,7 +185,7 @@ __global__ void __launch_bounds__(kBlock) k_bt_spmm(uint32_t n, uint32_t k, cons
 }
 
 // R = B - Y (R may be null); out = { Σ b², Σ (b - y)² } per column
-__global__ void __launch_bounds__(kBlock) k_bt_residual(uint32_t n, uint32_t k, const double* __restrict__ B,
+__global__ void __launch_bounds__(kRBlock) k_bt_residual(uint32_t n, uint32_t k, const double* __restrict__ B,
                                                         const double* __restrict__ Y, double* __restrict__ R,
                                                         BSlot slot) {
     const int lane = threadIdx.x & 31;
@@ -192,7 +209,7 @@ __global__ void __launch_bounds__(kBlock) k_bt_residual(uint32_t n, uint32_t k, 
 }
 
 // out = { Σ a b } per column
-__global__ void __launch_bounds__(kBlock) k_bt_dot(uint32_t n, uint32_t k, const double* __restrict__ A,
+__global__ void __launch_bounds__(kRBlock) k_bt_dot(uint32_t n, uint32_t k, const double* __restrict__ A,
                                                    const double* __restrict__ B, BSlot slot) {
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -209,7 +226,7 @@ __global__ void __launch_bounds__(kBlock) k_bt_dot(uint32_t n, uint32_t k, const
 }
 
 // Active columns: c = (w.v)/(d.v); d = w - c d.  Out: Σ d r per column (frozen columns keep d).
-__global__ void __launch_bounds__(kBlock) k_bt_fcg_direction(uint32_t n, uint32_t k, const double* __restrict__ W,
+__global__ void __launch_bounds__(kRBlock) k_bt_fcg_direction(uint32_t n, uint32_t k, const double* __restrict__ W,
                                                              double* __restrict__ D, const double* __restrict__ R,
                                                              const double* __restrict__ wv,
                                                              const double* __restrict__ dv,
@@ -247,7 +264,7 @@ __global__ void __launch_bounds__(kBlock) k_bt_fcg_direction(uint32_t n, uint32_
 }
 
 // Active columns: a = (d.r)/(d.v); x += a d; r -= a v.  Out: Σ r² per column.
-__global__ void __launch_bounds__(kBlock) k_bt_fcg_step(uint32_t n, uint32_t k, double* __restrict__ X,
+__global__ void __launch_bounds__(kRBlock) k_bt_fcg_step(uint32_t n, uint32_t k, double* __restrict__ X,
                                                         double* __restrict__ R, const double* __restrict__ D,
                                                         const double* __restrict__ V, const double* __restrict__ dr,
                                                         const double* __restrict__ dv, const int* __restrict__ active,
@@ -388,6 +405,11 @@ int bt_grid(const Handle& h, uint32_t n) {
     long cap = (long)h.info.sms * 4;
     if (want < 1) want = 1;
     return (int)(want < cap ? want : cap);
+}
+// blocks of the reducing kernels
+int bt_reduce_grid(const Handle& h, uint32_t n) {
+    const long want = std::max(1l, ((long)n + kRWarps - 1) / kRWarps);
+    return (int)std::min(want, (long)h.info.sms);
 }
 
 }  // namespace
@@ -535,15 +557,15 @@ void batched_apply(Handle& h, uint32_t k, const double* in_d, double* out_d, uin
 static void spmm(Handle& h, BatchWork& w, uint32_t k, const double* X, double* Y, int ndot = 0,
                  const double* Z = nullptr, const double* Q = nullptr, int slot = 0) {
     const uint32_t n = h.A.n;
-    const int g = bt_grid(h, n);
+    const int g = ndot == 0 ? bt_grid(h, n) : bt_reduce_grid(h, n);
     cudaStream_t s = h.stream;
     if (ndot == 0)
         k_bt_spmm<0><<<g, kBlock, 0, s>>>(n, k, h.A.rowptr.get(), h.A.col.get(), h.A.val.get(), X, Y, Z, Q, w.slot(0));
     else if (ndot == 1)
-        k_bt_spmm<1><<<g, kBlock, 0, s>>>(n, k, h.A.rowptr.get(), h.A.col.get(), h.A.val.get(), X, Y, Z, Q,
+        k_bt_spmm<1><<<g, kRBlock, 0, s>>>(n, k, h.A.rowptr.get(), h.A.col.get(), h.A.val.get(), X, Y, Z, Q,
                                           w.slot(slot));
     else
-        k_bt_spmm<2><<<g, kBlock, 0, s>>>(n, k, h.A.rowptr.get(), h.A.col.get(), h.A.val.get(), X, Y, Z, Q,
+        k_bt_spmm<2><<<g, kRBlock, 0, s>>>(n, k, h.A.rowptr.get(), h.A.col.get(), h.A.val.get(), X, Y, Z, Q,
                                           w.slot(slot));
     PRISM_LAUNCHED();
 }
@@ -558,7 +580,7 @@ void batched_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t k, const d
     double *B = w.B.get(), *X = w.X.get(), *R = w.R.get(), *W = w.W.get(), *D = w.D.get(), *V = w.V.get(),
            *Y = w.Y.get();
     double* sc = w.sc.get();
-    const int g = bt_grid(h, n);
+    const int g = bt_reduce_grid(h, n);
     const size_t nk = (size_t)n * k;
     uint32_t applies = 0, spmvs = 0;
     auto precond = [&]() {
@@ -575,14 +597,14 @@ void batched_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t k, const d
     // R = B - A X ; Σ b²
     spmm(h, w, k, X, Y);
     ++spmvs;
-    k_bt_residual<<<g, kBlock, 0, s>>>(n, k, B, Y, R, w.slot(BS_BB));
+    k_bt_residual<<<g, kRBlock, 0, s>>>(n, k, B, Y, R, w.slot(BS_BB));
     PRISM_LAUNCHED();
     precond();
     PRISM_CUDA(cudaMemcpyAsync(D, W, nk * sizeof(double), cudaMemcpyDeviceToDevice, s));
     // V = A D ; Σ v·d, Σ d·r
     spmm(h, w, k, D, V, 2, D, R, BS_DV);
     ++spmvs;
-    k_bt_fcg_step<<<g, kBlock, 0, s>>>(n, k, X, R, D, V, sc + BS_DR * kBK, sc + BS_DV * kBK, w.active.get(),
+    k_bt_fcg_step<<<g, kRBlock, 0, s>>>(n, k, X, R, D, V, sc + BS_DR * kBK, sc + BS_DV * kBK, w.active.get(),
                                        w.slot(BS_RR));
     PRISM_LAUNCHED();
     PRISM_CUDA(cudaMemcpyAsync(w.pinned, sc, kBScalars * kBK * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -620,21 +642,21 @@ void batched_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t k, const d
         }
         if (flexible) precond();
         else PRISM_CUDA(cudaMemcpyAsync(W, R, nk * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        k_bt_dot<<<g, kBlock, 0, s>>>(n, k, W, V, w.slot(BS_WV));
+        k_bt_dot<<<g, kRBlock, 0, s>>>(n, k, W, V, w.slot(BS_WV));
         PRISM_LAUNCHED();
-        k_bt_fcg_direction<<<g, kBlock, 0, s>>>(n, k, W, D, R, sc + BS_WV * kBK, sc + BS_DV * kBK, w.active.get(),
+        k_bt_fcg_direction<<<g, kRBlock, 0, s>>>(n, k, W, D, R, sc + BS_WV * kBK, sc + BS_DV * kBK, w.active.get(),
                                                 w.slot(BS_DR2));
         PRISM_LAUNCHED();
         spmm(h, w, k, D, V, 1, D, nullptr, BS_DV);
         ++spmvs;
-        k_bt_fcg_step<<<g, kBlock, 0, s>>>(n, k, X, R, D, V, sc + BS_DR2 * kBK, sc + BS_DV * kBK, w.active.get(),
+        k_bt_fcg_step<<<g, kRBlock, 0, s>>>(n, k, X, R, D, V, sc + BS_DR2 * kBK, sc + BS_DV * kBK, w.active.get(),
                                            w.slot(BS_RR));
         PRISM_LAUNCHED();
     }
     // true FP64 residuals
     spmm(h, w, k, X, Y);
     ++spmvs;
-    k_bt_residual<<<g, kBlock, 0, s>>>(n, k, B, Y, nullptr, w.slot(BS_BB));
+    k_bt_residual<<<g, kRBlock, 0, s>>>(n, k, B, Y, nullptr, w.slot(BS_BB));
     PRISM_LAUNCHED();
     launch_bt_unpack(s, h, n, k, ld, X, X_d);
     PRISM_CUDA(cudaEventRecord(h.ev1, s));

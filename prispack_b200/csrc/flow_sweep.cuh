@@ -35,9 +35,9 @@
 // serves them all, groups of CTAs take the columns. Us a sweep, level order before: IC 192^2,
 // 64 columns 4,208, now 311; AMSED 95x71 FP64, 13 columns 485 to 1,540, now 31.
 //
-// Measured against the streamed rounds (us an M^-1 apply): IC 64^2 FP64 150 against 334, IC
-// 512^2 FP64 1,052 against 2,948, ILUT 61x53x47 with float values 388 against 950 (level
-// order), AMSED 64^3 FP64 1,670 against 2,200, AMSED 128^3 with float arithmetic 4,476
+// Measured against the streamed rounds (us an M^-1 apply): IC 64^2 FP64 135 against 334, IC
+// 512^2 FP64 1,088 against 2,948, ILUT 61x53x47 with float values 371 against 950 (level
+// order), AMSED 64^3 FP64 1,557 against 2,200, AMSED 128^3 with float arithmetic 4,510
 // against 5,140.
 //
 // Progress: a task waits for earlier levels of its slab, held by warps that are ahead of it
@@ -451,43 +451,31 @@ static __global__ void __launch_bounds__(kFlowThreads, 1) k_sweep_flow(const Flo
             const uint32_t h1 = __ldg(a.halo_ptr + b + 1);
             constexpr uint32_t S = 32 * kFlowHaloWarps;
             uint32_t i = __ldg(a.halo_ptr + b) + (uint32_t)(warp - (int)kFlowWorkers) * 32 + (uint32_t)lane;
-            // U entries of the list in flight a lane, and the next U known
-            constexpr int U = N == 1 ? 4 : (N == 2 ? 2 : 1);
-            uint2 e[U], nx[U];
-            uint32_t at[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                e[u] = i + S * u < h1 ? __ldg(a.halo + i + S * u) : make_uint2(kFlowNone, 0);
-                nx[u] = i + S * (u + U) < h1 ? __ldg(a.halo + i + S * (u + U)) : make_uint2(kFlowNone, 0);
-                at[u] = i + S * (u + 2 * U);
-            }
+            // One entry of the list a lane and the next one known: four in flight a lane cost more
+            // registers and a longer way round the loop, which is what a value that is not there
+            // yet waits for (sweeps of 64^2 to 50^3: 2 to 5% slower)
+            uint2 e = i < h1 ? __ldg(a.halo + i) : make_uint2(kFlowNone, 0);
+            uint2 nx = i + S < h1 ? __ldg(a.halo + i + S) : make_uint2(kFlowNone, 0);
+            i += 2 * S;
             unsigned idle = 0;
-            bool more = true;
+            bool more = e.x != kFlowNone;
             while (__any_sync(0xFFFFFFFFu, more)) {
-                Acc v[U][N];
-                bool ok[U], some = false;
-                more = false;
+                Acc v[N];
+                bool some = false, ok = true;
                 // no branch between the loads: all are in flight at once
+                const FlowWord<Acc>* w = word_of(more ? e.x : 0u);
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const FlowWord<Acc>* w = word_of(e[u].x != kFlowNone ? e[u].x : 0u);
-                    ok[u] = true;
-#pragma unroll
-                    for (int j = 0; j < N; ++j) {
-                        const bool in = FlowWord<Acc>::get(w + j, v[u][j], epoch);
-                        ok[u] = in && ok[u];
-                    }
+                for (int j = 0; j < N; ++j) {
+                    const bool in = FlowWord<Acc>::get(w + j, v[j], epoch);
+                    ok = in && ok;
                 }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (ok[u] && e[u].x != kFlowNone) {
-                        store(xs + e[u].y * sb, v[u]);
-                        e[u] = nx[u];
-                        nx[u] = at[u] < h1 ? __ldg(a.halo + at[u]) : make_uint2(kFlowNone, 0);
-                        at[u] += U * S;
-                        some = true;
-                    }
-                    more = more || e[u].x != kFlowNone;
+                if (ok && more) {
+                    store(xs + e.y * sb, v);
+                    e = nx;
+                    nx = i < h1 ? __ldg(a.halo + i) : make_uint2(kFlowNone, 0);
+                    i += S;
+                    some = true;
+                    more = e.x != kFlowNone;
                 }
                 if (__any_sync(0xFFFFFFFFu, some)) {
                     idle = 0;

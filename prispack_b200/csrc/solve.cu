@@ -26,10 +26,12 @@ constexpr int kSpmvG = 1, kSpmvU = 2;                  // k_spmv: lanes per row,
 // suits short rows such as stencils, a group of lanes per row longer ones
 // Rows of a dataflow slab the tuner tries.  More slabs share a wavefront's rows among more SMs
 // and let a CTA take its next slab while the wavefront is elsewhere; fewer pay fewer hand-overs
-// from slab to slab (about 1 us each).  Measured (us an M^-1 apply, 1024 / 2048 / 4096 rows):
-// IC 512^2 FP64 1590 / 1269 / 1052, IC 40^3 FP64 437 / 473 / 580, AMSED 128^3 with float
-// arithmetic 4971 / 4476 / 5649.
-constexpr uint32_t kFlowSlabRows[3] = {1024, 2048, 4096};
+// from slab to slab (about 1 us each).  Measured (us an M^-1 apply, 512 / 1024 / 2048 / 4096
+// rows): IC 64^2 FP64 135 / 147 / 148 / 150, IC 512^2 FP64 2388 / 1759 / 1272 / 1088, IC 40^3
+// FP64 443 / 431 / 483 / 567, AMSED 64^3 FP64 1601 / 1726 / 2055 / 2682, GMSLR 50^3 with float
+// arithmetic 805 / 856 / 904 / 1020, AMSED 128^3 with float arithmetic 6483 / 5283 / 4563 / 5387.
+// With 256 rows the first is 153 and only AMSED 64^3 gains (1500).
+constexpr uint32_t kFlowSlabRows[4] = {512, 1024, 2048, 4096};
 // Rows of a slab of a block sweep: as many slabs as let the few CTAs of a group keep up with the
 // wavefront (512^2, k = 64, 2 columns: 5,266 us with 2,048 rows, 3,047 with 4,096; 192^2: 682 with
 // 1,024, 805 with 2,048).
@@ -877,8 +879,8 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
             cand.push_back({LAYOUT_FLOW, paired, h.info.flow_rows});
             return;
         }
-        for (uint32_t rows : kFlowSlabRows)  // small sweeps: one size, the others are within 3% (64^2: 151-152 us)
-            if (rows == kFlowSlabRows[0] || s.n > 16 * kFlowSlabRows[0]) cand.push_back({LAYOUT_FLOW, paired, rows});
+        for (uint32_t rows : kFlowSlabRows)  // small sweeps: the smallest size (64^2: 8% faster than the others)
+            if (rows == kFlowSlabRows[0] || s.n > 32 * kFlowSlabRows[0]) cand.push_back({LAYOUT_FLOW, paired, rows});
     };
     if (pp && h.info.stream_pair == 2) {  // paired where it fits
         streamed(true);

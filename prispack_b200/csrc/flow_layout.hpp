@@ -42,7 +42,7 @@
 
 namespace prism {
 
-constexpr uint32_t kFlowWorkers = 12;
+constexpr uint32_t kFlowWorkers = 13;
 // Named barriers in turn over a slab's levels.  A worker that waits for level l did its task
 // before at a level >= l - kFlowWorkers, whose barrier is done, so no barrier is taken up
 // again before it opened as long as there are at least kFlowWorkers of them.

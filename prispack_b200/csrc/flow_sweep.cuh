@@ -12,19 +12,23 @@
 //    in a slot of its own that holds a sentinel until the value is there.  No slot is used
 //    twice within a slab, so nothing has to be waited for before a write, and a reader
 //    needs no flag.
-//  - kFlowWorkers warps take the tasks in turn.  A warp sums the front of its task, whose
+//  - kFlowWorkers warps take the tasks in turn.  A task takes a warp some 1,700 cycles, 256
+//    instructions that mostly wait for one another, so every warp counts, and 16 are what
+//    128 registers a thread leave.  13 and three for the halo: IC 512^2 FP64 1,034 us an
+//    apply, FCG with AMSED on 64^3 91.9 ms, FGMRES with GMSLR on 50^3 30.1 ms; 12 and four
+//    1,070, 91.1, 31.3; 14 and two 1,004, 93.5, 29.3.  A warp sums the front of its task, whose
 //    values are mostly there, while the others finish the levels before; the level itself
 //    opens with a named barrier on which only the workers of two neighbouring levels meet
 //    (a hand-over of 93 cycles; polling the last values takes 2 to 3 times that, and
 //    polling warps slow down the one that the chain waits for).  Only then come the four
 //    tail values, their multiply-adds, the result's store and the next hand-over.
-//  - Four lanes a row: short tasks, so that 12 warps keep up with the chain (a lane a row:
+//  - Four lanes a row: short tasks, so that the workers keep up with the chain (a lane a row:
 //    0.26 us a level on 3D factors against 0.19).
 //  - Records come by plain 16-byte loads one chunk ahead into registers, from lines brought
 //    into L2 12 KB ahead; bulk copies into shared memory cost the worker more (a proxy fence
 //    waits for its global stores: 540 cycles a chunk).
 //  - Values that other slabs read go into an exchange array as {value, epoch} in one 8- or
-//    16-byte word; four warps a CTA copy the slab's halo from it into its slots.  The epoch
+//    16-byte word; three warps a CTA copy the slab's halo from it into its slots.  The epoch
 //    counts the sweeps of the layout, so nothing is marked before a sweep, the output can
 //    be the input, and a sweep that was given up leaves nothing that the next could take
 //    for its own.
@@ -36,8 +40,8 @@
 // 64 columns 4,208, now 311; AMSED 95x71 FP64, 13 columns 485 to 1,540, now 31.
 //
 // Measured against the streamed rounds (us an M^-1 apply): IC 64^2 FP64 135 against 334, IC
-// 512^2 FP64 1,088 against 2,948, ILUT 61x53x47 with float values 371 against 950 (level
-// order), AMSED 64^3 FP64 1,557 against 2,200, AMSED 128^3 with float arithmetic 4,510
+// 512^2 FP64 1,034 against 2,948, ILUT 61x53x47 with float values 365 against 950 (level
+// order), AMSED 64^3 FP64 1,600 against 2,200, AMSED 128^3 with float arithmetic 4,500
 // against 5,140.
 //
 // Progress: a task waits for earlier levels of its slab, held by warps that are ahead of it
@@ -54,7 +58,7 @@
 
 namespace prism {
 
-constexpr int kFlowHaloWarps = 4;
+constexpr int kFlowHaloWarps = 3;
 constexpr int kFlowThreads = 32 * ((int)kFlowWorkers + kFlowHaloWarps);
 constexpr uint32_t kFlowFixedSmem = 128;    // "leave" word, then the value slots
 constexpr unsigned kFlowPolls = 1024;       // polls of a value slot between looks at the clock

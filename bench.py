@@ -52,8 +52,8 @@ METRIC = "time-to-1e-10 rel. residual, mixed FP32-factor / FP64-Krylov, 1 B200"
 AMSED = dict(levels=3, lanczos_steps=64, low_rank=32, eig_bound=0.8, lowrank_type=0, lanczos_type=0, reorder=0)
 SEED = 2024
 # DRAM bytes / algorithmic bytes of the streamed sweep kernel's level-0 lower sweep (one ncu capture on the
-# 96^3 case, profiles/k_sweep_stream_fp32apply_level0_lower_96cube.md), applied to each launch's algorithmic bytes
-TRAFFIC_RATIO = {"level-order": 181.2 / 183.6, "stream": 256.4 / 183.6}
+# 96^3 case, profiles/k_sweep_flow_fp32apply_level0_lower_96cube.md), applied to each launch's algorithmic bytes
+TRAFFIC_RATIO = {"level-order": 181.2 / 183.6, "stream": 253.4 / 183.6}
 TRAFFIC_SOURCE = ("ncu capture of the level-0 lower sweep at 96^3 (183.6 MB algorithmic): DRAM read + write "
                   "bytes / algorithmic bytes, scaled to this launch")
 # the reference library's timing build (oracle/Makefile FAST_FLAGS)
@@ -778,8 +778,8 @@ def main():
             s0 = torch.cuda.Event(enable_timing=True)
             s1 = torch.cuda.Event(enable_timing=True)
             s0.record(stream)
-            # the whole sweep as the apply runs it: marking the output pending (and, for the
-            # streamed layout, staging the right-hand side into its round records), then the sweep
+            # the whole sweep as the apply runs it: marking the output pending where the kernel
+            # needs that (the dataflow sweep does not), then the sweep
             S.sweep_device(sw, vin, vout, 1)
             s1.record(stream)
             torch.cuda.synchronize()

@@ -99,7 +99,7 @@ static __global__ void __launch_bounds__(kBlock) k_bk_sub(uint64_t count, const 
 // ---------------------------------------------------------------------------
 // Block partials of W^T X for rank columns q and block columns c: thread (g, c) with
 // g = threadIdx.x / 64 sums q = g, g + 4, ... over the block's rows (grid-stride by
-// blocks of 64 rows); the last block adds the partials in block order and scales by H.
+// tiles of kLrTile rows); the last block adds the partials in block order and scales by H.
 // Rows a block takes at a time, and at most one block an SM: with 64 rows a block, six blocks
 // worked on the 371 rows below the first level of a 95 x 71 grid (13 columns: 33 us).
 constexpr uint32_t kLrTile = 8;

@@ -19,8 +19,8 @@
 //
 // The factor values then go into every device layout of the preconditioner's
 // sweeps through maps built once from the factor's pattern: the level-order and
-// slab layouts' value and diagonal arrays, and the streamed layout's round
-// records (coefficients, and each row's diagonal or its reciprocal).
+// slab layouts' value and diagonal arrays, the dataflow layout's chunks and diagonals,
+// the rounds' records (coefficients, and each row's diagonal or its reciprocal).
 #include <algorithm>
 #include <cmath>
 #include <memory>

@@ -21,7 +21,7 @@ struct DeviceInfo {
     int sms = 148;
     int sweep_blocks_per_sm = 1;   // co-resident k_sweep blocks (cooperative launch bound)
     int max_smem_optin = 0;        // bytes of dynamic shared memory one block may opt into
-    int sweep_kernel = 0;          // 0: autotune per sweep, 1: global level order, 2: slab-blocked, 3: streamed rounds
+    int sweep_kernel = 0;          // 0: autotune per sweep, 1: global level order, 2: slab-blocked, 3: streamed (dataflow or rounds)
     uint32_t slab_min_rows = 2048; // smallest slab (small systems use fewer CTAs)
     uint32_t slab_max_rows = 1u << 30;  // largest slab (default: what shared memory holds)
     uint32_t stream_min_rows = 1024;    // smallest streamed slab (small systems use fewer CTAs)

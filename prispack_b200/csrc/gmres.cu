@@ -312,7 +312,7 @@ struct CycleGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint32_t nodes = 0;
-    // the key: the preconditioner object, every buffer the step touches, the sizes
+    // the key: the preconditioner's device arrays (its uid), every buffer the step touches, the sizes
     uint64_t precond_uid = 0;
     const void* bufs[7] = {};
     uint32_t n = 0, restart = 0;
@@ -471,7 +471,7 @@ void gmres_solve(Handle& h, const prism_solve_opts& o, const double* b, double* 
     uint32_t applies = 0, spmvs = 0, syncs = 0, body_nodes = 0;
 
     // one restart cycle as a graph, unless the caller asks for plain launches; the graph of an
-    // earlier solve is replayed when it was captured from the same preconditioner object and
+    // earlier solve is replayed when it was captured from the same preconditioner arrays and
     // buffers
     CycleGraph* graph = nullptr;
     if (o.launch_mode != PRISM_LAUNCH_STREAM) {

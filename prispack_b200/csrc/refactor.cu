@@ -542,8 +542,10 @@ void TriangularPrecond::refactor() {
     cudaStream_t st = h_.stream;
     const bool ldlt = F.kind == 3;
     // A paired sweep's coefficients combine several factor entries, which the value maps
-    // below cannot rebuild: such sweeps are tuned again without pairing first.
+    // below cannot rebuild: such sweeps are tuned again without pairing first.  Their old
+    // device arrays go, so what was captured from them (a GMRES cycle graph) must not run again.
     if (!rf_ && (lower_.paired || upper_.paired)) {
+        renew_uid();
         if (F.fp32) {
             if (lower_.paired) tune_sweep(h_, lower_, F.lower32, F.apply32, false);
             if (upper_.paired) tune_sweep(h_, upper_, F.upper32, F.apply32, false);

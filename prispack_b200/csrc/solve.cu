@@ -964,6 +964,7 @@ namespace {
 std::atomic<uint64_t> g_precond_uid{0};
 }
 Precond::Precond() : uid(++g_precond_uid) {}
+void Precond::renew_uid() { uid = ++g_precond_uid; }
 
 TriangularPrecond::TriangularPrecond(Handle& h, std::shared_ptr<const HostFactor> f) : h_(h), f_(std::move(f)) {
     // the streamed kernel may run the sweeps paired (refactor() tunes them again unpaired)

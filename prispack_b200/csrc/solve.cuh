@@ -146,9 +146,10 @@ class Precond {
   public:
     Precond();
     virtual ~Precond() = default;
-    // distinct for every preconditioner object of the process (never reused), so that work
-    // captured from one (a GMRES cycle graph) is never replayed against another
-    const uint64_t uid;
+    // distinct for every set of device arrays a preconditioner of the process applies from
+    // (never reused), so that work captured from one (a GMRES cycle graph) is never replayed
+    // against another: the object's first, and another one before its arrays are replaced
+    uint64_t uid;
     virtual int kind() const = 0;
     virtual uint64_t mnnz() const = 0;
     // out = M^{-1} in; in != out not required.
@@ -182,6 +183,9 @@ class Precond {
         (void)which; (void)n; (void)nnz; (void)rowptr; (void)col; (void)val; (void)diag;
         return 9;
     }
+
+  protected:
+    void renew_uid();
 };
 
 struct Handle;

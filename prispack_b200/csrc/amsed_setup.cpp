@@ -3,14 +3,13 @@
 // reference's setup for the same partition; the Lanczos quantities agree to
 // rounding (their tridiagonal eigen-decomposition is this file's own).
 #include "amsed_setup.hpp"
+#include "host_threads.hpp"
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <limits>
 #include <numeric>
 #include <random>
-#include <thread>
 
 extern "C" int64_t prism_graph_bisect(int32_t n, const int32_t* xadj, const int32_t* adjncy, int32_t* part);
 
@@ -591,25 +590,6 @@ void tridiag_eig(int m, const double* d_in, const double* e_in, double* mu, doub
 // ============================================================================
 // Host applies of the partial preconditioner
 // ============================================================================
-// fn(i) for i in [0, count) on up to `threads` host threads (the items are independent:
-// the results do not depend on the thread count)
-template <typename F>
-void host_parallel_for(uint32_t count, unsigned threads, F&& fn) {
-    threads = std::min<unsigned>(threads, count);
-    if (threads <= 1) {
-        for (uint32_t i = 0; i < count; ++i) fn(i);
-        return;
-    }
-    std::atomic<uint32_t> next{0};
-    std::vector<std::thread> pool;
-    for (unsigned t = 0; t < threads; ++t)
-        pool.emplace_back([&] {
-            for (uint32_t i = next++; i < count; i = next++) fn(i);
-        });
-    for (auto& th : pool) th.join();
-}
-unsigned host_threads() { return std::max(1u, std::min(std::thread::hardware_concurrency(), 16u)); }
-
 template <typename Low>
 void amsed_block_solve_host(const AmsedSetup<Low>& S, int level, double* x) {
     const AmsedLevel<Low>& L = S.levels[level];

@@ -1,35 +1,15 @@
 // Host side of the dataflow sweep layout (flow_layout.hpp).
 #include "flow_layout.hpp"
+#include "host_threads.hpp"
 
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <cstdlib>
 #include <cstring>
-#include <thread>
 #include <unordered_map>
 
 namespace prism {
 namespace {
-
-// f(b) for b in [0, n) on host threads
-template <typename F>
-void on_threads(uint32_t n, F&& f) {
-    unsigned hc = std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
-    if (const char* e = std::getenv("PRISM_LAYOUT_THREADS")) hc = (unsigned)std::max(1, std::atoi(e));
-    hc = std::min<unsigned>(hc, n);
-    if (hc <= 1) {
-        for (uint32_t b = 0; b < n; ++b) f(b);
-        return;
-    }
-    std::atomic<uint32_t> next{0};
-    std::vector<std::thread> pool;
-    for (unsigned t = 0; t < hc; ++t)
-        pool.emplace_back([&] {
-            for (uint32_t b = next++; b < n; b = next++) f(b);
-        });
-    for (auto& t : pool) t.join();
-}
 
 struct SlabPlan {
     std::vector<uint32_t> pos;        // positions of the sweep, in (level, row) order
@@ -93,7 +73,7 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
     for (auto& x : pub) x.store(0, std::memory_order_relaxed);
     std::atomic<bool> fits{true};
     std::atomic<uint32_t> most{0};
-    on_threads(ns, [&](uint32_t b) {
+    host_parallel_for(ns, layout_threads(), [&](uint32_t b) {
         SlabPlan& P = plan[b];
         const uint32_t m = (uint32_t)P.pos.size();
         std::unordered_map<uint32_t, uint32_t> seen;
@@ -189,7 +169,7 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
         order->ecoef.assign(order->eptr[n], 0.0);
     }
     if (coef_map) coef_map->assign(s.val.size() * 2, 0);
-    on_threads(ns, [&](uint32_t b) {
+    host_parallel_for(ns, layout_threads(), [&](uint32_t b) {
         const SlabPlan& P = plan[b];
         std::unordered_map<uint32_t, uint32_t> hs;
         for (size_t i = 0; i < P.halo.size(); ++i) {

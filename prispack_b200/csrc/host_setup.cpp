@@ -1,6 +1,7 @@
 // Host-side setup: model problems, bit-exact incomplete factorisations and the
 // exact integer level schedules used by the device sweeps.
 #include "host_setup.hpp"
+#include "host_threads.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -8,7 +9,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
-#include <thread>
 #include <type_traits>
 
 namespace prism {
@@ -484,9 +484,7 @@ void pair_sweep(const Sweep<Low>& s, Sweep<Low>& out, PairMap& m) {
         std::vector<Low> cv;
         std::vector<double> coef;
     };
-    unsigned hc = std::max(1u, std::thread::hardware_concurrency());
-    if (const char* e = std::getenv("PRISM_LAYOUT_THREADS")) hc = (unsigned)std::max(1, std::atoi(e));
-    const uint32_t T = n < 65536 ? 1u : std::min<uint32_t>(std::min(hc, 16u), n);
+    const uint32_t T = n < 65536 ? 1u : std::min<uint32_t>(std::min(layout_threads(), 16u), n);
     std::vector<Chunk> parts(T);
     auto work = [&](uint32_t t) {
         Chunk& c = parts[t];
@@ -542,13 +540,7 @@ void pair_sweep(const Sweep<Low>& s, Sweep<Low>& out, PairMap& m) {
             for (uint32_t j : deps) slot[j] = -1;
         }
     };
-    if (T == 1) {
-        work(0);
-    } else {
-        std::vector<std::thread> pool;
-        for (uint32_t t = 0; t < T; ++t) pool.emplace_back(work, t);
-        for (auto& th : pool) th.join();
-    }
+    host_parallel_for(T, T, work);
     std::vector<uint32_t> rp((size_t)n + 1, 0), ci;
     std::vector<Low> cv;
     m.ptr.assign((size_t)n + 1, 0);
@@ -1201,11 +1193,9 @@ bool stream_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint
     };
     // the slabs on a few host threads, each with its own scratch
     {
-        unsigned hc = std::max(1u, std::thread::hardware_concurrency());
-        if (const char* e = std::getenv("PRISM_LAYOUT_THREADS")) hc = (unsigned)std::max(1, std::atoi(e));
-        const unsigned T = num_ctas < 8 ? 1u : std::min<unsigned>(std::min(hc, 16u), num_ctas);
+        const unsigned T = num_ctas < 8 ? 1u : std::min<unsigned>(std::min(layout_threads(), 16u), num_ctas);
         std::atomic<uint32_t> next{0};
-        auto worker = [&]() {
+        auto worker = [&](uint32_t) {
             Scratch sc;
             sc.seen.assign(n, kNone);
             sc.last_use.assign(n, -1);
@@ -1213,13 +1203,7 @@ bool stream_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint
             sc.slot_in.assign(n, kNone);
             for (uint32_t b = next++; b < num_ctas; b = next++) lay_slab(b, sc, parts[b]);
         };
-        if (T == 1) {
-            worker();
-        } else {
-            std::vector<std::thread> pool;
-            for (unsigned t = 0; t < T; ++t) pool.emplace_back(worker);
-            for (auto& th : pool) th.join();
-        }
+        host_parallel_for(T, T, worker);
     }
     // assembly, slab by slab
     for (uint32_t b = 0; b < num_ctas; ++b) {

@@ -519,18 +519,20 @@ void launch_bt_unpack(cudaStream_t st, const Handle& h, uint32_t n, uint32_t k, 
 // ============================================================================
 void TriangularPrecond::apply_batched(cudaStream_t st, uint32_t k, const double* in, double* out) {
     const uint32_t n = h_.A.n;
-    const uint32_t cols = block_columns(k, n);
+    const uint32_t cols = block_columns(k, n), w = block_width_index(cols);
     auto copy = [&](DevSweep& mine, bool lower) -> const DevSweep& {
         if (mine.n != n) {
-            if (f_->fp32) mine.upload_block(lower ? f_->lower32 : f_->upper32, h_.info, cols, h_.stream);
-            else mine.upload_block(lower ? f_->lower64 : f_->upper64, h_.info, cols, h_.stream);
-            refresh_block_copy(mine, lower);  // after a device refactorisation: its values
+            DevSweep d;
+            if (f_->fp32) d.upload_block(lower ? f_->lower32 : f_->upper32, h_.info, cols, h_.stream);
+            else d.upload_block(lower ? f_->lower64 : f_->upper64, h_.info, cols, h_.stream);
+            refresh_block_copy(d, w, lower);  // after a device refactorisation: its values
+            mine = std::move(d);
         }
         mine.block_workspace(k, st);
         return mine;
     };
-    const DevSweep& lo = copy(lower_bk_[block_width_index(cols)], true);
-    const DevSweep& up = copy(upper_bk_[block_width_index(cols)], false);
+    const DevSweep& lo = copy(lower_bk_[w], true);
+    const DevSweep& up = copy(upper_bk_[w], false);
     const size_t nk = (size_t)n * k;
     if (tmpk_.size() < nk) tmpk_.alloc(nk);
     if (!lo.self_filling()) launch_bt_fill(st, h_, nk, tmpk_.get());

@@ -376,6 +376,7 @@ int rf_grid(const Handle& h, uint64_t items) {
 struct SweepValueMap {
     DevBuf<uint32_t> cdst, csrc, ddst, dsrc;
     uint32_t ncoef = 0, ndiag = 0;
+    bool built = false;
 };
 
 struct RefactorState {
@@ -389,7 +390,8 @@ struct RefactorState {
     DevBuf<double> lt64, D;
     DevBuf<int> status;       // [status, first bad column]
     DevBuf<unsigned> bad;     // first out-of-range map entry: [coefficients, diagonals]
-    SweepValueMap lower, upper, block;
+    SweepValueMap lower, upper;
+    SweepValueMap lower_bk[kBlockWidths], upper_bk[kBlockWidths];  // of the copies for the block sweeps
     bool refactored = false;  // the device factor differs from the host one
 };
 void refactor_release(RefactorState* r) { delete r; }
@@ -403,6 +405,7 @@ void upload_map(SweepValueMap& M, const std::vector<uint32_t>& cd, const std::ve
     M.csrc.upload(cs.data(), cs.size(), st);
     M.ddst.upload(dd.data(), dd.size(), st);
     M.dsrc.upload(ds.data(), ds.size(), st);
+    M.built = true;
 }
 
 // The map of device sweep d, uploaded from host sweep s (idx: the same sweep with factor
@@ -696,33 +699,42 @@ void TriangularPrecond::refactor() {
         apply_map<double>(h_, st, lower_, R.lower, R.lt64.get(), lt_n, D, ic, R.bad.get());
         apply_map<double>(h_, st, upper_, R.upper, R.lt64.get(), lt_n, D, ic, R.bad.get());
     }
+    for (uint32_t w = 0; w < kBlockWidths; ++w) {
+        if (lower_bk_[w].n) refresh_block_copy(lower_bk_[w], R.lower_bk[w], true);
+        if (upper_bk_[w].n) refresh_block_copy(upper_bk_[w], R.upper_bk[w], false);
+    }
     check_maps(R, st, "the sweeps");
-    // the copies of the block solves are uploaded again on their next use, with the new
-    // values (refresh_block_copy)
-    for (DevSweep& d : lower_bk_) d.release();
-    for (DevSweep& d : upper_bk_) d.release();
     R.refactored = true;
     PRISM_CUDA(cudaStreamSynchronize(st));
 }
 
-void TriangularPrecond::refresh_block_copy(DevSweep& d, bool lower) {
-    if (!rf_ || !rf_->refactored) return;
+// The refactored values into a copy for the block sweeps; its map is built once.  (Copies uploaded
+// again after each refactorisation, laid out twice on the host: IC 64^3, 8 columns, refactorisation
+// and block apply 1,308 ms.)
+void TriangularPrecond::refresh_block_copy(DevSweep& d, SweepValueMap& M, bool lower) {
     const HostFactor& F = *f_;
     RefactorState& R = *rf_;
     cudaStream_t st = h_.stream;
-    Sweep<double> ilo, iup;
-    factor_index_sweeps(F, ilo, iup);
-    SweepValueMap& M = R.block;
     const uint64_t lt_n = F.f0.col.size();
-    PRISM_CUDA(cudaMemsetAsync(R.bad.get(), 0, 2 * sizeof(unsigned), st));
-    if (F.fp32) {
-        build_map<float>(d, lower ? F.lower32 : F.upper32, lower ? ilo : iup, M, st);
-        apply_map<float>(h_, st, d, M, R.lt32.get(), lt_n, R.D.get(), F.kind == 1, R.bad.get());
-    } else {
-        build_map<double>(d, lower ? F.lower64 : F.upper64, lower ? ilo : iup, M, st);
-        apply_map<double>(h_, st, d, M, R.lt64.get(), lt_n, R.D.get(), F.kind == 1, R.bad.get());
+    if (!M.built) {
+        Sweep<double> ilo, iup;
+        factor_index_sweeps(F, ilo, iup);
+        const Sweep<double>& idx = lower ? ilo : iup;
+        if (F.fp32) build_map<float>(d, lower ? F.lower32 : F.upper32, idx, M, st);
+        else build_map<double>(d, lower ? F.lower64 : F.upper64, idx, M, st);
     }
-    check_maps(R, st, "a block copy");
+    if (F.fp32) apply_map<float>(h_, st, d, M, R.lt32.get(), lt_n, R.D.get(), F.kind == 1, R.bad.get());
+    else apply_map<double>(h_, st, d, M, R.lt64.get(), lt_n, R.D.get(), F.kind == 1, R.bad.get());
+}
+
+// A copy for the block sweeps uploaded from the host factor: nothing to do until the device has
+// refactored it.
+void TriangularPrecond::refresh_block_copy(DevSweep& d, uint32_t width, bool lower) {
+    if (!rf_ || !rf_->refactored) return;
+    RefactorState& R = *rf_;
+    PRISM_CUDA(cudaMemsetAsync(R.bad.get(), 0, 2 * sizeof(unsigned), h_.stream));
+    refresh_block_copy(d, lower ? R.lower_bk[width] : R.upper_bk[width], lower);
+    check_maps(R, h_.stream, "a block copy");
 }
 
 int TriangularPrecond::export_refactored(int which, uint32_t* n, uint64_t* nnz, uint32_t* rowptr, uint32_t* col,

@@ -190,6 +190,7 @@ class Precond {
 
 struct Handle;
 struct RefactorState;              // device refactorisation of an IC / ILDLT factor (refactor.cu)
+struct SweepValueMap;
 void refactor_release(RefactorState* r);
 
 // IC / ILDLT / ILUT: two sweeps on the device (ILDLT's D^{-1} is folded into
@@ -216,7 +217,8 @@ class TriangularPrecond : public Precond {
   private:
     int export_refactored(int which, uint32_t* n, uint64_t* nnz, uint32_t* rowptr, uint32_t* col, double* val,
                           double* diag) const;
-    void refresh_block_copy(DevSweep& d, bool lower);
+    void refresh_block_copy(DevSweep& d, SweepValueMap& map, bool lower);
+    void refresh_block_copy(DevSweep& d, uint32_t width, bool lower);
     Handle& h_;
     std::shared_ptr<const HostFactor> f_;
     DevSweep lower_, upper_;

@@ -6,10 +6,15 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
-#include <unordered_map>
 
 namespace prism {
 namespace {
+
+// An entry of a row: {level (halo rows later) << 32 | row read, stored entry, slot}.
+struct Item {
+    uint64_t key;
+    uint32_t k, slot;
+};
 
 struct SlabPlan {
     std::vector<uint32_t> pos;        // positions of the sweep, in (level, row) order
@@ -17,6 +22,49 @@ struct SlabPlan {
     std::vector<uint32_t> chunks;     // chunks of each task
     std::vector<uint32_t> level;      // first task of each level of the slab, and the end
     std::vector<std::pair<uint32_t, uint32_t>> halo;  // {row, slot}
+    std::vector<uint32_t> up;         // the slabs it reads
+};
+
+// Rows of other slabs -> their slots in the slab in work: open addressing, at most half full.
+// Entries of the slabs before are told apart by their tag, so nothing is cleared between slabs.
+class HaloSlots {
+  public:
+    HaloSlots() : tab_(1024, Entry{0, 0}) {}
+    void start() {
+        ++tag_;
+        count_ = 0;
+    }
+    // the slot of `row`: `fresh` where it has none yet
+    uint32_t put(uint32_t row, uint32_t fresh) {
+        Entry& e = find(row);
+        if (e.key >> 32 == tag_) return e.slot;
+        e = Entry{(uint64_t)tag_ << 32 | row, fresh};
+        if (++count_ * 2 > tab_.size()) grow();
+        return fresh;
+    }
+
+  private:
+    struct Entry {
+        uint64_t key;
+        uint32_t slot;
+    };
+    // the entry of `row`, or the free one where it goes
+    Entry& find(uint32_t row) {
+        const uint64_t key = (uint64_t)tag_ << 32 | row;
+        for (uint64_t i = (row * 0x9E3779B97F4A7C15ull) >> 32;; ++i) {
+            Entry& e = tab_[i & (tab_.size() - 1)];
+            if (e.key == key || e.key >> 32 != tag_) return e;
+        }
+    }
+    void grow() {
+        std::vector<Entry> old(tab_.size() * 2, Entry{0, 0});
+        old.swap(tab_);
+        for (const Entry& e : old)
+            if (e.key >> 32 == tag_) find((uint32_t)e.key) = e;
+    }
+    std::vector<Entry> tab_;
+    uint32_t tag_ = 0;
+    size_t count_ = 0;
 };
 
 }  // namespace
@@ -34,35 +82,13 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
     const uint32_t E = entries ? entries : (s.val.size() <= 12 * (uint64_t)n ? 4 : 8), RB = Q * E * (2 + vb);
     out.entries = E;
     auto tail_bytes = [](uint32_t m) { return flow_tail_bytes(m, vb); };
-    std::vector<uint32_t> owner(n), slot(n);
-    // Slabs from upstream to downstream, by their depth in the graph of slabs: independent
-    // blocks advance side by side where a CTA takes several slabs.
-    std::vector<uint32_t> number(ns);
-    {
-        std::vector<uint32_t> depth(ns, 0), at(ns);
-        for (uint32_t i = 0; i < ns; ++i) {
-            const uint32_t b = s.lower ? i : ns - 1 - i;
-            for (uint32_t r = start[b]; r < start[b + 1]; ++r) owner[r] = b;
-        }
-        std::vector<uint32_t> pos_of(n);
-        for (uint32_t p = 0; p < n; ++p) pos_of[s.order[p]] = p;
-        for (uint32_t i = 0; i < ns; ++i) {
-            const uint32_t b = s.lower ? i : ns - 1 - i;
-            for (uint32_t r = start[b]; r < start[b + 1]; ++r)
-                for (uint32_t k = s.rowptr[pos_of[r]]; k < s.rowptr[pos_of[r] + 1]; ++k)
-                    if (owner[s.col[k]] != b) depth[b] = std::max(depth[b], depth[owner[s.col[k]]] + 1);
-            at[i] = b;
-        }
-        std::stable_sort(at.begin(), at.end(), [&](uint32_t x, uint32_t y) { return depth[x] < depth[y]; });
-        for (uint32_t i = 0; i < ns; ++i) number[at[i]] = i;
-    }
-    auto slab_of = [&](uint32_t b) { return number[b]; };
-    for (uint32_t b = 0; b < ns; ++b) {
+    for (uint32_t b = 0; b < ns; ++b)
         if (start[b + 1] - start[b] >= max_slots) return false;
-        for (uint32_t r = start[b]; r < start[b + 1]; ++r) owner[r] = slab_of(b);
-    }
+    std::vector<uint32_t> owner(n), slot(n);
+    for (uint32_t b = 0; b < ns; ++b)
+        for (uint32_t r = start[b]; r < start[b + 1]; ++r) owner[r] = b;
     std::vector<SlabPlan> plan(ns);
-    for (uint32_t b = 0; b < ns; ++b) plan[slab_of(b)].pos.reserve(start[b + 1] - start[b]);
+    for (uint32_t b = 0; b < ns; ++b) plan[b].pos.reserve(start[b + 1] - start[b]);
     for (uint32_t p = 0; p < n; ++p) {
         const uint32_t r = s.order[p];
         SlabPlan& P = plan[owner[r]];
@@ -72,47 +98,77 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
     std::vector<std::atomic<uint8_t>> pub(n);
     for (auto& x : pub) x.store(0, std::memory_order_relaxed);
     std::atomic<bool> fits{true};
-    std::atomic<uint32_t> most{0};
-    host_parallel_for(ns, layout_threads(), [&](uint32_t b) {
-        SlabPlan& P = plan[b];
-        const uint32_t m = (uint32_t)P.pos.size();
-        std::unordered_map<uint32_t, uint32_t> seen;
-        uint32_t longest = 0, used = m + 1;
-        auto close = [&]() { P.chunks.push_back(std::max(1u, (longest + Q * E - 1) / (Q * E))); };
-        for (uint32_t i = 0; i < m; ++i) {
-            const uint32_t p = P.pos[i];
-            const bool opens = i == 0 || s.level[s.order[p]] != s.level[s.order[P.pos[i - 1]]];
-            if (opens || i - P.task.back() == kFlowRows) {
-                if (i) close();
-                if (opens) P.level.push_back((uint32_t)P.task.size());
-                P.task.push_back(i);
-                longest = 0;
+    std::atomic<uint32_t> most{0}, next{0};
+    const uint32_t T = std::min<uint32_t>(layout_threads(), ns);
+    host_parallel_for(T, T, [&](uint32_t) {
+        HaloSlots seen;
+        for (uint32_t b = next++; b < ns && fits; b = next++) {
+            SlabPlan& P = plan[b];
+            const uint32_t m = (uint32_t)P.pos.size(), r0 = start[b], r1 = start[b + 1];
+            seen.start();
+            uint32_t longest = 0, used = m + 1;
+            auto close = [&]() { P.chunks.push_back(std::max(1u, (longest + Q * E - 1) / (Q * E))); };
+            for (uint32_t i = 0; i < m && used <= max_slots; ++i) {
+                const uint32_t p = P.pos[i];
+                const bool opens = i == 0 || s.level[s.order[p]] != s.level[s.order[P.pos[i - 1]]];
+                if (opens || i - P.task.back() == kFlowRows) {
+                    if (i) close();
+                    if (opens) P.level.push_back((uint32_t)P.task.size());
+                    P.task.push_back(i);
+                    longest = 0;
+                }
+                uint32_t own = 0;
+                for (uint32_t k = s.rowptr[p]; k < s.rowptr[p + 1]; ++k) {
+                    const uint32_t c = s.col[k];
+                    if (c >= r0 && c < r1) {
+                        ++own;
+                    } else if (used <= max_slots && seen.put(c, used) == used) {
+                        P.halo.push_back({c, used++});
+                        pub[c].store(1, std::memory_order_relaxed);
+                    }
+                }
+                longest = std::max(longest, s.rowptr[p + 1] - s.rowptr[p] - std::min(own, kFlowTail));
             }
-            uint32_t own = 0;
-            for (uint32_t k = s.rowptr[p]; k < s.rowptr[p + 1]; ++k) {
-                const uint32_t c = s.col[k];
-                own += owner[c] == b;
-                if (owner[c] == b || !seen.emplace(c, used).second) continue;
-                P.halo.push_back({c, used++});
-                pub[c].store(1, std::memory_order_relaxed);
+            if (used > max_slots) {
+                fits = false;
+                return;
             }
-            longest = std::max(longest, s.rowptr[p + 1] - s.rowptr[p] - std::min(own, kFlowTail));
+            close();
+            P.level.push_back((uint32_t)P.task.size());
+            P.task.push_back(m);
+            uint32_t cur = most.load();
+            while (cur < used && !most.compare_exchange_weak(cur, used)) {
+            }
+            // values arrive by level
+            std::sort(P.halo.begin(), P.halo.end(), [&](const auto& x, const auto& y) {
+                return s.level[x.first] != s.level[y.first] ? s.level[x.first] < s.level[y.first] : x.first < y.first;
+            });
+            for (uint32_t c : P.chunks)
+                if (c > 0xFFu) fits = false;
+            P.up.reserve(P.halo.size());
+            for (const auto& h : P.halo)
+                if (P.up.empty() || P.up.back() != owner[h.first]) P.up.push_back(owner[h.first]);
+            std::sort(P.up.begin(), P.up.end());
+            P.up.erase(std::unique(P.up.begin(), P.up.end()), P.up.end());
         }
-        close();
-        P.level.push_back((uint32_t)P.task.size());
-        P.task.push_back(m);
-        if (used > max_slots) fits = false;
-        uint32_t cur = most.load();
-        while (cur < used && !most.compare_exchange_weak(cur, used)) {
-        }
-        // values arrive by level
-        std::sort(P.halo.begin(), P.halo.end(), [&](const auto& x, const auto& y) {
-            return s.level[x.first] != s.level[y.first] ? s.level[x.first] < s.level[y.first] : x.first < y.first;
-        });
-        for (uint32_t c : P.chunks)
-            if (c > 0xFFu) fits = false;
     });
     if (!fits) return false;
+    // Slabs from upstream to downstream, by their depth in the graph of slabs: independent
+    // blocks advance side by side where a CTA takes several slabs.
+    std::vector<uint32_t> range_of(ns);  // slab number -> its rows' range in `start`
+    {
+        std::vector<uint32_t> depth(ns, 0);
+        for (uint32_t i = 0; i < ns; ++i) {
+            const uint32_t b = s.lower ? i : ns - 1 - i;
+            for (uint32_t u : plan[b].up) depth[b] = std::max(depth[b], depth[u] + 1);
+            range_of[i] = b;
+        }
+        std::stable_sort(range_of.begin(), range_of.end(),
+                         [&](uint32_t x, uint32_t y) { return depth[x] < depth[y]; });
+        std::vector<SlabPlan> sorted(ns);
+        for (uint32_t i = 0; i < ns; ++i) sorted[i] = std::move(plan[range_of[i]]);
+        plan.swap(sorted);
+    }
     out.slots = most;
     // exchange entries, in the order the rows are computed
     std::vector<uint32_t> entry(n, kFlowNone);
@@ -144,7 +200,7 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
         out.halo_ptr[b + 1] = out.halo_ptr[b] + (uint32_t)P.halo.size();
     }
     if (chunk > 0xFFFFFFFFull || bytes / vb > 0xFFFFFFFFull) return false;  // u32 positions (coef_map)
-    out.chunks.assign(bytes, 0);
+    out.chunks.alloc(bytes);
     out.hdr.assign((size_t)out.tasks * kFlowRows * 4, 0);
     out.dg.assign((size_t)out.tasks * kFlowRows, 1.0);
     out.dg_pos.assign(n, 0);
@@ -169,18 +225,15 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
         order->ecoef.assign(order->eptr[n], 0.0);
     }
     if (coef_map) coef_map->assign(s.val.size() * 2, 0);
-    host_parallel_for(ns, layout_threads(), [&](uint32_t b) {
+    auto lay = [&](uint32_t b, HaloSlots& hs, std::vector<Item>& it) {
         const SlabPlan& P = plan[b];
-        std::unordered_map<uint32_t, uint32_t> hs;
+        const uint32_t r0 = start[range_of[b]], r1 = start[range_of[b] + 1];
+        hs.start();
         for (size_t i = 0; i < P.halo.size(); ++i) {
-            hs.emplace(P.halo[i].first, P.halo[i].second);
+            hs.put(P.halo[i].first, P.halo[i].second);
             out.halo[2 * (out.halo_ptr[b] + i)] = entry[P.halo[i].first];
             out.halo[2 * (out.halo_ptr[b] + i) + 1] = P.halo[i].second;
         }
-        struct Item {
-            uint32_t key, dep, k;
-        };
-        std::vector<Item> it;
         // the workers of each level, as bits; the level and barrier counts of each task
         const uint32_t nl = (uint32_t)P.level.size() - 1;
         std::vector<uint32_t> who(nl + 1, 0), meet((size_t)P.chunks.size(), 0), lev(P.chunks.size());
@@ -196,6 +249,7 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
         for (uint32_t w = 0; w < kFlowWorkers; ++w) {
             const uint32_t* q = &out.warp[((size_t)b * kFlowWorkers + w) * 8];
             uint64_t start16 = (uint64_t)q[4] * 16;
+            if (q[5]) std::memset(&out.chunks[start16], 0, (size_t)q[5] * 16);
             uint32_t task = q[1];
             for (size_t t = w; t < P.chunks.size(); t += kFlowWorkers, ++task) {
                 const uint32_t nc = P.chunks[t], m = P.task[t + 1] - P.task[t];
@@ -216,24 +270,30 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
                     out.dg[(size_t)task * kFlowRows + j8] = recip ? 1.0 / d : d;
                     out.dg_pos[r] = task * kFlowRows + j8;
                     it.clear();
-                    for (uint32_t k = s.rowptr[p]; k < s.rowptr[p + 1]; ++k)
-                        it.push_back({s.level[s.col[k]] + (owner[s.col[k]] == b ? 0u : kFlowHaloLag), s.col[k], k});
-                    std::sort(it.begin(), it.end(), [](const Item& x, const Item& y) {
-                        return x.key != y.key ? x.key < y.key : (x.dep != y.dep ? x.dep < y.dep : x.k < y.k);
-                    });
+                    for (uint32_t k = s.rowptr[p]; k < s.rowptr[p + 1]; ++k) {
+                        const uint32_t c = s.col[k];
+                        const bool own = c >= r0 && c < r1;
+                        it.push_back({(uint64_t)(s.level[c] + (own ? 0u : kFlowHaloLag)) << 32 | c, k,
+                                      own ? slot[c] : hs.put(c, 0)});
+                    }
+                    std::sort(it.begin(), it.end(),
+                              [](const Item& x, const Item& y) { return x.key != y.key ? x.key < y.key : x.k < y.k; });
                     // the latest rows of the slab to the end, the others' order kept
+                    const uint32_t all = (uint32_t)it.size();
                     uint32_t tail = 0;
-                    std::vector<Item> last;
-                    for (size_t j = it.size(); j-- > 0 && tail < kFlowTail;)
-                        if (owner[it[j].dep] == b) {
-                            last.push_back(it[j]);
-                            it.erase(it.begin() + j);
-                            ++tail;
-                        }
-                    const uint32_t front = (uint32_t)it.size();
-                    it.insert(it.end(), last.rbegin(), last.rend());
-                    for (uint32_t j = 0; j < it.size(); ++j) {
-                        const uint16_t sl = (uint16_t)(owner[it[j].dep] == b ? slot[it[j].dep] : hs[it[j].dep]);
+                    Item last[kFlowTail];
+                    uint32_t to = all;  // where the entries kept are moved to, from the end
+                    for (uint32_t j = all; j-- > 0;) {
+                        const uint32_t c = (uint32_t)it[j].key;
+                        if (tail < kFlowTail && c >= r0 && c < r1) last[tail++] = it[j];
+                        else it[--to] = it[j];
+                    }
+                    // entries [to, all) are the front now; to == tail
+                    const uint32_t front = all - tail;
+                    for (uint32_t j = 0; j < all; ++j) {
+                        const Item& en = j < front ? it[tail + j] : last[all - 1 - j];
+                        const uint32_t dep = (uint32_t)en.key;
+                        const uint16_t sl = (uint16_t)en.slot;
                         uint64_t at;  // where the coefficient goes
                         if (j < front) {
                             // position, its lane, chunk and place in the chunk
@@ -243,29 +303,35 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
                             std::memcpy(&out.chunks[base + (lane * E + c) * 2], &sl, 2);
                             at = base + 2 * E * Q * m + (uint64_t)(c * vb / 16) * 16 * Q * m + lane * 16 + c * vb % 16;
                             if (order) {
-                                order->edep[order->eptr[r] + e] = it[j].dep;
-                                order->ecoef[order->eptr[r] + e] = (double)s.val[it[j].k];
+                                order->edep[order->eptr[r] + e] = dep;
+                                order->ecoef[order->eptr[r] + e] = (double)s.val[en.k];
                             }
                         } else {
-                            const uint32_t c = kFlowTail - ((uint32_t)it.size() - j);
+                            const uint32_t c = kFlowTail - (all - j);
                             const uint64_t base = start16 + (uint64_t)nc * m * RB;
                             std::memcpy(&out.chunks[base + 4 * vb * m + j8 * 8 + c * 2], &sl, 2);
                             at = base + (uint64_t)(c * vb / 16) * 16 * m + j8 * 16 + c * vb % 16;
                             if (order) {
-                                order->kdep[r * kFlowTail + c] = it[j].dep;
-                                order->kcoef[r * kFlowTail + c] = (double)s.val[it[j].k];
+                                order->kdep[r * kFlowTail + c] = dep;
+                                order->kcoef[r * kFlowTail + c] = (double)s.val[en.k];
                             }
                         }
-                        std::memcpy(&out.chunks[at], &s.val[it[j].k], vb);
+                        std::memcpy(&out.chunks[at], &s.val[en.k], vb);
                         if (coef_map) {
-                            (*coef_map)[2 * (size_t)it[j].k] = (uint32_t)(at / vb);
-                            (*coef_map)[2 * (size_t)it[j].k + 1] = it[j].k;
+                            (*coef_map)[2 * (size_t)en.k] = (uint32_t)(at / vb);
+                            (*coef_map)[2 * (size_t)en.k + 1] = en.k;
                         }
                     }
                 }
                 start16 += (uint64_t)nc * m * RB + tail_bytes(m);
             }
         }
+    };
+    next = 0;
+    host_parallel_for(T, T, [&](uint32_t) {
+        HaloSlots hs;
+        std::vector<Item> it;
+        for (uint32_t b = next++; b < ns; b = next++) lay(b, hs, it);
     });
     return true;
 }

@@ -36,6 +36,7 @@
 // Slabs are numbered from upstream to downstream.
 #pragma once
 
+#include <memory>
 #include <string>
 
 #include "host_setup.hpp"
@@ -54,10 +55,27 @@ PRISM_HD constexpr uint32_t flow_tail_bytes(uint32_t m, uint32_t vb) { return (m
 constexpr uint32_t kFlowNone = 0xFFFFFFFFu;
 constexpr uint32_t kFlowHaloLag = 8;
 
+// Bytes that alloc leaves untouched: each slab's thread clears and fills its own.
+class FlowBytes {
+  public:
+    void alloc(size_t count) {
+        p_.reset(new uint8_t[count]);
+        n_ = count;
+    }
+    const uint8_t* data() const { return p_.get(); }
+    size_t size() const { return n_; }
+    uint8_t& operator[](size_t i) { return p_[i]; }
+    const uint8_t& operator[](size_t i) const { return p_[i]; }
+
+  private:
+    std::unique_ptr<uint8_t[]> p_;
+    size_t n_ = 0;
+};
+
 struct FlowLayout {
     uint32_t entries = 0;              // E
     uint32_t slabs = 0, slots = 0, published = 0, tasks = 0;  // slots: of the slab that needs most
-    std::vector<uint8_t> chunks;
+    FlowBytes chunks;
     std::vector<uint32_t> hdr, warp, halo_ptr, halo;
     std::vector<double> dg;
     std::vector<uint32_t> dg_pos;  // per row: its entry of dg

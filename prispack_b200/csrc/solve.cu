@@ -4,6 +4,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <future>
+#include <limits>
 
 #include "../../include/prism_solve.h"
 #include "kernels.cuh"
@@ -31,7 +32,8 @@ constexpr int kSpmvG = 1, kSpmvU = 2;                  // k_spmv: lanes per row,
 // FP64 443 / 431 / 483 / 567, AMSED 64^3 FP64 1601 / 1726 / 2055 / 2682, GMSLR 50^3 with float
 // arithmetic 805 / 856 / 904 / 1020, AMSED 128^3 with float arithmetic 6483 / 5283 / 4563 / 5387.
 // With 256 rows the first is 153 and only AMSED 64^3 gains (1500).
-constexpr uint32_t kFlowSlabRows[4] = {512, 1024, 2048, 4096};
+constexpr int kFlowSizes = 4;
+constexpr uint32_t kFlowSlabRows[kFlowSizes] = {512, 1024, 2048, 4096};
 // Rows of a slab of a block sweep: as many slabs as let the few CTAs of a group keep up with the
 // wavefront (512^2, k = 64, 2 columns: 5,266 us with 2,048 rows, 3,047 with 4,096; 192^2: 682 with
 // 1,024, 805 with 2,048).
@@ -537,16 +539,13 @@ void DevSweep::release() {
 }
 
 template <typename Low>
-StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair) {
+StreamPlan plan_stream(const Sweep<Low>& s0, const DeviceInfo& info, bool acc32) {
     // One persistent CTA per SM (fewer for small sweeps); shared memory holds the
     // round table, the value slots and, in what is left, the ring the round
     // records stream through.
     StreamPlan P;
-    const uint32_t nn = sweep.n;
+    const uint32_t nn = s0.n;
     if (nn == 0) return P;
-    Sweep<Low> ps;
-    if (pair) pair_sweep<Low>(sweep, ps, P.pm);
-    const Sweep<Low>& s0 = pair ? ps : sweep;
     const uint32_t ctas_req = stream_slab_count(nn, (uint32_t)info.sms, info.stream_min_rows);
     const std::vector<uint32_t> start = slab_ranges<Low>(s0, ctas_req);
     const uint64_t smem = (uint64_t)info.max_smem_optin;
@@ -578,7 +577,6 @@ StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc
     }
     if (!fits) return P;
     P.ok = true;
-    P.paired = pair;
     P.fp32 = std::is_same<Low, float>::value;
     P.a32 = a32;
     P.n = s0.n;
@@ -593,18 +591,14 @@ StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc
     P.nnz = s0.val.size();
     return P;
 }
-template StreamPlan plan_stream<double>(const Sweep<double>&, const DeviceInfo&, bool, bool);
-template StreamPlan plan_stream<float>(const Sweep<float>&, const DeviceInfo&, bool, bool);
+template StreamPlan plan_stream<double>(const Sweep<double>&, const DeviceInfo&, bool);
+template StreamPlan plan_stream<float>(const Sweep<float>&, const DeviceInfo&, bool);
 
 template <typename Low>
-StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows,
-                     uint32_t cols) {
+StreamPlan plan_flow(const Sweep<Low>& s0, const DeviceInfo& info, bool acc32, uint32_t rows, uint32_t cols) {
     StreamPlan P;
-    const uint32_t nn = sweep.n;
+    const uint32_t nn = s0.n;
     if (nn == 0) return P;
-    Sweep<Low> ps;
-    if (pair) pair_sweep<Low>(sweep, ps, P.pm);
-    const Sweep<Low>& s0 = pair ? ps : sweep;
     P.a32 = acc32 && std::is_same<Low, float>::value;
     P.cols = cols;
     P.slot_bytes = (P.a32 ? 4 : 8) * std::max(cols, 1u);
@@ -617,7 +611,6 @@ StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32
         if (nn / want < 64) return P;
     }
     P.ok = P.flow = true;
-    P.paired = pair;
     P.fp32 = std::is_same<Low, float>::value;
     P.n = s0.n;
     P.num_levels = s0.num_levels;
@@ -628,8 +621,8 @@ StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32
     P.nnz = s0.val.size();
     return P;
 }
-template StreamPlan plan_flow<double>(const Sweep<double>&, const DeviceInfo&, bool, bool, uint32_t, uint32_t);
-template StreamPlan plan_flow<float>(const Sweep<float>&, const DeviceInfo&, bool, bool, uint32_t, uint32_t);
+template StreamPlan plan_flow<double>(const Sweep<double>&, const DeviceInfo&, bool, uint32_t, uint32_t);
+template StreamPlan plan_flow<float>(const Sweep<float>&, const DeviceInfo&, bool, uint32_t, uint32_t);
 
 void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
     const StreamLayout& L = P.L;
@@ -643,11 +636,11 @@ void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
     str_ctas_req = P.ctas_req;
     str_nnz = P.nnz;
     str_smem = P.smem;
-    if (P.paired) {
+    if (P.pm) {
         paired = true;
-        pair_ptr.upload(P.pm.ptr.data(), P.pm.ptr.size(), st);
-        pair_dep.upload(P.pm.dep.data(), P.pm.dep.size(), st);
-        pair_coef.upload(P.pm.coef.data(), P.pm.coef.size(), st);
+        pair_ptr.upload(P.pm->ptr.data(), P.pm->ptr.size(), st);
+        pair_dep.upload(P.pm->dep.data(), P.pm->dep.size(), st);
+        pair_coef.upload(P.pm->coef.data(), P.pm->coef.size(), st);
         if (pair_dep.size() == 0) pair_dep.alloc(1);  // valid pointers for the prep
         if (pair_coef.size() == 0) pair_coef.alloc(1);
     }
@@ -713,8 +706,7 @@ void DevSweep::commit_stream(StreamPlan&& P, cudaStream_t st) {
 template <typename Low>
 void DevSweep::upload_block(const Sweep<Low>& s, const DeviceInfo& info, uint32_t cols, cudaStream_t st) {
     if (s.n > 0) {
-        StreamPlan P = plan_flow<Low>(s, info, false, false, info.flow_rows ? info.flow_rows : block_slab_rows(s.n),
-                                         cols);
+        StreamPlan P = plan_flow<Low>(s, info, false, info.flow_rows ? info.flow_rows : block_slab_rows(s.n), cols);
         if (P.ok) {
             if (s.op == SWEEP_DIV || s.op == SWEEP_PREDIV) {
                 P.diag.resize(s.n);
@@ -739,10 +731,11 @@ void DevSweep::block_workspace(uint32_t k, cudaStream_t st) {
 }
 
 template <typename Low>
-bool DevSweep::upload(const Sweep<Low>& sweep, const DeviceInfo& info, int lay, cudaStream_t st, bool pair) {
+bool DevSweep::upload(const Sweep<Low>& sweep, const DeviceInfo& info, int lay, cudaStream_t st) {
     if (lay == LAYOUT_STREAM || lay == LAYOUT_FLOW) {
-        StreamPlan P = lay == LAYOUT_FLOW ? plan_flow<Low>(sweep, info, acc32, pair, info.flow_rows ? info.flow_rows : kFlowSlabRows[0])
-                                          : plan_stream<Low>(sweep, info, acc32, pair);
+        StreamPlan P = lay == LAYOUT_FLOW
+                           ? plan_flow<Low>(sweep, info, acc32, info.flow_rows ? info.flow_rows : kFlowSlabRows[0])
+                           : plan_stream<Low>(sweep, info, acc32);
         if (!P.ok) return false;
         commit_stream(std::move(P), st);
         return true;
@@ -846,116 +839,151 @@ void stream_sweep_run(int device, const Sweep<Low>& s, bool acc32, uint32_t num_
 template void stream_sweep_run<double>(int, const Sweep<double>&, bool, uint32_t, const double*, double*);
 template void stream_sweep_run<float>(int, const Sweep<float>&, bool, uint32_t, const double*, double*);
 
-// Sweep-kernel autotuner: uploads the sweep in each device layout in turn
+// Sweep-kernel autotuner: uploads the sweep in one device layout after another
 // (level order for k_sweep, slabs for k_sweep_slab, dataflow slabs for k_sweep_flow
 // or, where they do not fit, rounds for k_sweep_stream), times a few launches of
 // each, output marking included, on a fixed right-hand side with CUDA events, and
-// keeps the fastest.  Which
-// kernel wins depends on how many rows a wavefront holds and how far
-// dependencies reach.
+// keeps the fastest.  Which kernel wins depends on how many rows a wavefront holds
+// and how far dependencies reach.
+//
+// Single-precision arithmetic: only the streamed kernels have it (the other layouts,
+// where no streamed one fits, compute in double).  Slab sizes are climbed from one to its
+// neighbours, the sweep's time having one minimum over them (kFlowSlabRows), and the paired
+// sweep is laid out for its own minimum only where at the unpaired sweep's best size it is within
+// a quarter of it.  At most two layouts are in host memory, and the paired sweep, which is worked
+// out while the unpaired ones are timed (all sizes, paired and not, laid out at once held eight
+// layouts, 450 MB each for the level-0 sweep of 128^3 with float values, and four paired sweeps).
 template <typename Low>
 void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pair) {
     const int mode = h.info.sweep_kernel;
-    d.acc32 = acc32 && std::is_same<Low, float>::value;
+    const bool a32 = d.acc32 = acc32 && std::is_same<Low, float>::value;
     // Pairing keeps the arithmetic's precision class only where the derived coefficients are
     // stored in the arithmetic's own type: double values (FP64) or float values with float
     // arithmetic; float values with double arithmetic (<float,double>) stay unpaired.
-    const bool pp = pair && h.info.stream_pair != 0 && (d.acc32 || std::is_same<Low, double>::value);
-    if (s.n == 0) {
-        d.upload(s, h.info, LAYOUT_LEVEL, h.stream);
+    const bool pp = pair && h.info.stream_pair != 0 && (a32 || std::is_same<Low, double>::value);
+    const bool only_paired = pp && h.info.stream_pair == 2;  // paired where it fits
+    const bool any = mode == 0 && !a32 && !only_paired;      // every layout is a candidate
+    if (s.n == 0 || (mode != 0 && mode != 3 && !a32 && !only_paired)) {
+        d.upload(s, h.info, s.n != 0 && mode == 2 ? LAYOUT_SLAB : LAYOUT_LEVEL, h.stream);
         return;
     }
-    // candidates.  Single-precision arithmetic: only the streamed kernels have it (the other
-    // layouts, where no streamed one fits, compute in double).  The streamed kernel is the
-    // dataflow one; the rounds take the sweeps that do not fit it.
-    struct Cand {
-        int layout;
-        bool paired;
-        uint32_t rows;
+    struct Paired {
+        Sweep<Low> s;
+        PairMap m;
     };
-    std::vector<Cand> cand;
-    auto streamed = [&](bool paired) {
-        if (h.info.flow_rows) {
-            cand.push_back({LAYOUT_FLOW, paired, h.info.flow_rows});
-            return;
-        }
-        for (uint32_t rows : kFlowSlabRows)  // small sweeps: the smallest size (64^2: 8% faster than the others)
-            if (rows == kFlowSlabRows[0] || s.n > 32 * kFlowSlabRows[0]) cand.push_back({LAYOUT_FLOW, paired, rows});
-    };
-    if (pp && h.info.stream_pair == 2) {  // paired where it fits
-        streamed(true);
-    } else if (d.acc32 || mode == 3) {
-        streamed(false);
-        if (pp) streamed(true);
-    } else if (mode != 0) {
-        cand.push_back({mode == 2 ? LAYOUT_SLAB : LAYOUT_LEVEL, false, 0});
-    } else {
-        cand = {{LAYOUT_LEVEL, false, 0}, {LAYOUT_SLAB, false, 0}};
-        streamed(false);
-        if (pp) streamed(true);
-    }
-    if (cand.size() == 1 && cand[0].layout != LAYOUT_FLOW) {
-        d.upload(s, h.info, cand[0].layout, h.stream);
-        return;
-    }
+    std::future<Paired> pairing;
+    if (pp)
+        pairing = std::async([&s] {
+            Paired p;
+            pair_sweep<Low>(s, p.s, p.m);
+            return p;
+        });
     DevBuf<double> in(s.n), out(s.n);
     std::vector<double> rhs(s.n);
     for (uint32_t i = 0; i < s.n; ++i) rhs[i] = 1.0 + (double)(i % 7) * 0.125;
     in.upload(rhs.data(), s.n, h.stream);
-    cudaEvent_t e0, e1;
-    PRISM_CUDA(cudaEventCreate(&e0));
-    PRISM_CUDA(cudaEventCreate(&e1));
-    float best = 0.f;
-    int best_c = -1;
-    // the streamed candidates' host layouts are built concurrently
-    std::vector<std::future<StreamPlan>> plans(cand.size());
-    for (int c = 0; c < (int)cand.size(); ++c)
-        if (cand[c].layout == LAYOUT_FLOW) {
-            const bool a32 = d.acc32, first = cand[c].rows == kFlowSlabRows[0] || h.info.flow_rows != 0;
-            const Cand cc = cand[c];
-            plans[c] = std::async(std::launch::async, [&s, &h, a32, cc, first] {
-                StreamPlan P = plan_flow<Low>(s, h.info, a32, cc.paired, cc.rows);
-                if (!P.ok && first) P = plan_stream<Low>(s, h.info, a32, cc.paired);
-                return P;
-            });
+    struct Events {
+        cudaEvent_t e[2] = {};
+        ~Events() {
+            for (cudaEvent_t x : e)
+                if (x) cudaEventDestroy(x);
         }
+    } ev;
+    for (cudaEvent_t& x : ev.e) PRISM_CUDA(cudaEventCreate(&x));
+    constexpr float kNever = std::numeric_limits<float>::infinity();
+    float best = kNever;
     DevSweep kept;  // the fastest candidate so far, kept uploaded
-    for (int c = 0; c < (int)cand.size(); ++c) {
-        DevSweep t;
-        t.acc32 = d.acc32;
-        if (cand[c].layout == LAYOUT_FLOW) {
-            StreamPlan P = plans[c].get();
-            if (!P.ok) continue;
-            t.commit_stream(std::move(P), h.stream);
-        } else if (!t.upload(s, h.info, cand[c].layout, h.stream)) {
-            continue;
-        }
-        float tot = 0.f;
+    auto time = [&](DevSweep&& t) {
+        float least = kNever;
         for (int it = 0; it < 4; ++it) {
-            PRISM_CUDA(cudaEventRecord(e0, h.stream));
+            PRISM_CUDA(cudaEventRecord(ev.e[0], h.stream));
             launch_sweep_prepare(h, h.stream, t, in.get(), out.get());
             launch_sweep_kernel(h, h.stream, t, in.get(), out.get());
-            PRISM_CUDA(cudaEventRecord(e1, h.stream));
-            PRISM_CUDA(cudaEventSynchronize(e1));
+            PRISM_CUDA(cudaEventRecord(ev.e[1], h.stream));
+            PRISM_CUDA(cudaEventSynchronize(ev.e[1]));
             float ms = 0.f;
-            PRISM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            if (it > 0) tot += ms;  // first launch is a warm-up
+            PRISM_CUDA(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
+            if (it > 0) least = std::min(least, ms);  // first launch is a warm-up
         }
         h.check_status();
-        if (best_c < 0 || tot < best) {
-            best = tot;
-            best_c = c;
+        if (least < best) {
+            best = least;
             kept = std::move(t);
         }
+        return least;
+    };
+    auto plain = [&](int layout) {
+        DevSweep t;
+        t.acc32 = a32;
+        if (t.upload(s, h.info, layout, h.stream)) time(std::move(t));
+    };
+    // small sweeps: the smallest size (64^2: 8% faster than the others)
+    const bool climbs = !h.info.flow_rows && s.n > 32 * kFlowSlabRows[0];
+    const uint32_t only_rows = h.info.flow_rows ? h.info.flow_rows : kFlowSlabRows[0];
+    // the unpaired layouts that are needed in any case: on the host while the one before is timed
+    int size = 1;
+    uint32_t ahead_rows = 0;
+    std::future<StreamPlan> ahead;
+    auto lay_ahead = [&](uint32_t rows) {
+        ahead_rows = rows;
+        ahead = std::async([&s, &h, a32, rows] { return plan_flow<Low>(s, h.info, a32, rows); });
+    };
+    // the streamed layouts of sw, starting from kFlowSlabRows[at]; returns the best size
+    auto streamed = [&](const Sweep<Low>& sw, const PairMap* pm, int at) {
+        auto upload = [&](StreamPlan&& P) {
+            P.pm = pm;
+            DevSweep t;
+            t.acc32 = a32;
+            t.commit_stream(std::move(P), h.stream);
+            return time(std::move(t));
+        };
+        bool first = true;
+        auto flow = [&](uint32_t rows) {
+            StreamPlan P = rows == ahead_rows ? ahead.get() : plan_flow<Low>(sw, h.info, a32, rows);
+            ahead_rows = 0;
+            if (first && !pm && climbs) lay_ahead(kFlowSlabRows[at - 1]);
+            if (!P.ok && first) P = plan_stream<Low>(sw, h.info, a32);
+            // slabs that had to be split are those of a smaller size
+            const bool split = P.ok && P.flow && P.ctas_req > (s.n + rows - 1) / rows;
+            if (!P.ok || (split && !first)) return kNever;
+            first = false;
+            return upload(std::move(P));
+        };
+        if (!climbs) {
+            flow(only_rows);
+            return 0;
+        }
+        const float unpaired = best;
+        float here = flow(kFlowSlabRows[at]);
+        if (pm && here > 1.25f * unpaired) return at;
+        for (int step : {-1, 1}) {
+            const int from = at;
+            while (at + step >= 0 && at + step < kFlowSizes) {
+                const float t = flow(kFlowSlabRows[at + step]);
+                if (t >= here) break;
+                here = t;
+                at += step;
+            }
+            if (at != from) break;
+        }
+        return at;
+    };
+    if (!only_paired) lay_ahead(climbs ? kFlowSlabRows[size] : only_rows);
+    if (any) {
+        plain(LAYOUT_LEVEL);
+        plain(LAYOUT_SLAB);
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    if (best_c < 0) {  // nothing fitted (streamed layouts only): level order, double arithmetic
+    if (!only_paired) size = streamed(s, nullptr, size);
+    if (pairing.valid()) {
+        const Paired p = pairing.get();
+        streamed(p.s, &p.m, size);
+    }
+    if (best == kNever) {  // nothing fitted (streamed layouts only): level order, double arithmetic
         d.upload(s, h.info, LAYOUT_LEVEL, h.stream);
         return;
     }
     d = std::move(kept);
-    d.tuned_ms = best / 3.f;
+    d.tuned_ms = best;
 }
 template void tune_sweep<double>(Handle&, DevSweep&, const Sweep<double>&, bool, bool);
 template void tune_sweep<float>(Handle&, DevSweep&, const Sweep<float>&, bool, bool);

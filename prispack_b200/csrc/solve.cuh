@@ -62,27 +62,26 @@ struct DeviceCsr {
 enum SweepLayout : int { LAYOUT_LEVEL = 0, LAYOUT_SLAB = 1, LAYOUT_STREAM = 2, LAYOUT_FLOW = 3 };
 
 // One triangular sweep resident on the device (see build_sweep for the layout).
-// The host part of a streamed upload (pairing, layout, launch shape; no CUDA calls), which
+// The host part of a streamed upload (layout and launch shape; no CUDA calls), which
 // DevSweep::commit_stream uploads: the dataflow layout F (flow) or the rounds L.
 // ok false: the sweep does not fit.
 struct StreamPlan {
-    bool ok = false, paired = false, fp32 = false, a32 = false, flow = false;
+    bool ok = false, fp32 = false, a32 = false, flow = false;
     uint32_t cols = 0;             // of a block, per CTA (0: single vectors)
     std::vector<double> diag;      // blocks of dividing sweeps: the diagonal, by row
     StreamLayout L;
     FlowLayout F;
-    PairMap pm;
+    const PairMap* pm = nullptr;   // of a paired sweep (the caller's): its right-hand side map
     uint32_t n = 0, num_levels = 0;
     int op = 0;
     uint32_t ctas = 0, ctas_req = 0, slot_bytes = 0, cap = 0, ring = 0, smem = 0;
     uint64_t nnz = 0;
 };
 template <typename Low>
-StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair);
+StreamPlan plan_stream(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32);
 // rows: of a slab (fewer where a slab's rows and halo do not fit in shared memory)
 template <typename Low>
-StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, bool pair, uint32_t rows,
-                     uint32_t cols = 0);
+StreamPlan plan_flow(const Sweep<Low>& sweep, const DeviceInfo& info, bool acc32, uint32_t rows, uint32_t cols = 0);
 // the columns a CTA takes of a block of k, n rows
 uint32_t block_columns(uint32_t k, uint32_t n);
 constexpr uint32_t kBlockWidths = 3;  // 1, 2 or 4 columns a CTA
@@ -120,10 +119,9 @@ struct DevSweep {
     DevBuf<uint32_t> pair_ptr, pair_dep;
     DevBuf<double> pair_coef, pair_rhs;
     // Uploads the sweep in the given layout; false (nothing uploaded) when the
-    // layout does not fit the sweep (stream layout only).  pair: the streamed layout
-    // of the paired sweep (half the wavefronts; other layouts ignore it).
+    // layout does not fit the sweep (streamed layouts only).
     template <typename Low>
-    bool upload(const Sweep<Low>& s, const DeviceInfo& info, int layout, cudaStream_t st, bool pair = false);
+    bool upload(const Sweep<Low>& s, const DeviceInfo& info, int layout, cudaStream_t st);
     void commit_stream(StreamPlan&& plan, cudaStream_t st);
     // Uploads the sweep for blocks of columns, `cols` of them a CTA (block_columns): dataflow
     // slabs, level order where they do not fit.

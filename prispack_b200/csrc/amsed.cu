@@ -12,6 +12,7 @@
 // recursion.  All scratch is allocated once, at construction.
 #include <algorithm>
 #include <cstring>
+#include <functional>
 
 #include "amsed_block.cuh"
 #include "amsed_setup.hpp"
@@ -230,8 +231,9 @@ void AmsedPrecond::apply(cudaStream_t st, const double* in, double* out) {
 // ============================================================================
 // Block apply: k <= 64 interleaved columns (X[row * k + c])
 // ============================================================================
-void launch_bt_fill(cudaStream_t st, const Handle& h, uint64_t count, double* p);
-void launch_bt_sweep(const Handle& h, cudaStream_t st, const DevSweep& s, uint32_t k, const double* in, double* out);
+void run_block_sweep(const Handle& h, cudaStream_t st, const DevSweep& s, uint32_t k, const double* in, double* out);
+void choose_block_sweep(Handle& h, BlockSweep& B, const DevSweep& tuned, uint32_t k, uint32_t width, const double* in,
+                        double* out, const std::function<void(DevSweep&)>& upload_level);
 
 namespace {
 // float -> BF16, round to nearest even (NaN kept quiet)
@@ -264,22 +266,46 @@ void AmsedPrecond::prepare_block(uint32_t k) {
             if (a_->fp32) {
                 Sweep<float> lo, up;
                 level_sweeps<float>(*a_->s32, l, lo, up);
-                B.lower[wi].upload_block(lo, h_.info, cols, st);
-                B.upper[wi].upload_block(up, h_.info, cols, st);
+                B.lower.flow[wi].upload_block(lo, h_.info, cols, st);
+                B.upper.flow[wi].upload_block(up, h_.info, cols, st);
             } else {
                 Sweep<double> lo, up;
                 level_sweeps<double>(*a_->s64, l, lo, up);
-                B.lower[wi].upload_block(lo, h_.info, cols, st);
-                B.upper[wi].upload_block(up, h_.info, cols, st);
+                B.lower.flow[wi].upload_block(lo, h_.info, cols, st);
+                B.upper.flow[wi].upload_block(up, h_.info, cols, st);
             }
         }
         blv_width_ |= 1u << wi;
     }
     for (BlockLevel& B : blv_) {
-        B.lower[wi].block_workspace(k, st);
-        B.upper[wi].block_workspace(k, st);
+        B.lower.flow[wi].block_workspace(k, st);
+        B.upper.flow[wi].block_workspace(k, st);
     }
-    if (bk_ >= k) return;
+    if (bk_ < k) block_buffers(k);
+    if (blv_[0].lower.choice[k] != BlockSweep::UNTIMED) return;
+    PRISM_CUDA(cudaMemsetAsync(Xk_.get(), 0, (size_t)n_ * k * sizeof(double), st));
+    for (uint32_t l = nlev_; l-- > 0;)  // level 0, which tells that they are timed, last
+        for (bool lower : {false, true}) {
+            BlockLevel& B = blv_[l];
+            choose_block_sweep(h_, lower ? B.lower : B.upper, lower ? lv_[l].lower : lv_[l].upper, k, wi, Xk_.get(),
+                               sweep_tmpk_.get(), [&](DevSweep& d) {
+                                   if (a_->fp32) {
+                                       Sweep<float> lo, up;
+                                       level_sweeps<float>(*a_->s32, l, lo, up);
+                                       d.upload(lower ? lo : up, h_.info, LAYOUT_LEVEL, st);
+                                   } else {
+                                       Sweep<double> lo, up;
+                                       level_sweeps<double>(*a_->s64, l, lo, up);
+                                       d.upload(lower ? lo : up, h_.info, LAYOUT_LEVEL, st);
+                                   }
+                                   PRISM_CUDA(cudaStreamSynchronize(st));
+                               });
+        }
+}
+
+// The workspace of blocks of up to k columns.
+void AmsedPrecond::block_buffers(uint32_t k) {
+    cudaStream_t st = h_.stream;
     tensor_lowrank_ = a_->fp32;
     const bool first = bk_ == 0;
     size_t part64 = 1, part32 = 1, t64 = 1, t32 = 1;
@@ -343,14 +369,9 @@ void AmsedPrecond::block_solve_k(cudaStream_t st, int level, uint32_t k, const d
     if (L.nfac < L.nb && in != out)
         PRISM_CUDA(cudaMemcpyAsync(out + (size_t)L.nfac * k, in + (size_t)L.nfac * k,
                                    (size_t)(L.nb - L.nfac) * k * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    const uint64_t cnt = (uint64_t)L.nfac * k;
-    const DevSweep& lo = B.lower[block_width_index(block_columns(k, n_))];
-    const DevSweep& up = B.upper[block_width_index(block_columns(k, n_))];
-    if (!lo.self_filling()) launch_bt_fill(st, h_, cnt, sweep_tmpk_.get());
-    if (in != out && !up.self_filling()) launch_bt_fill(st, h_, cnt, out);
-    launch_bt_sweep(h_, st, lo, k, in, sweep_tmpk_.get());
-    if (in == out && !up.self_filling()) launch_bt_fill(st, h_, cnt, out);
-    launch_bt_sweep(h_, st, up, k, sweep_tmpk_.get(), out);
+    const uint32_t wi = block_width_index(block_columns(k, n_));
+    run_block_sweep(h_, st, B.lower.of(k, wi, L.lower), k, in, sweep_tmpk_.get());
+    run_block_sweep(h_, st, B.upper.of(k, wi, L.upper), k, sweep_tmpk_.get(), out);
 }
 
 // x2 += W (H o (W^T xc)) on k columns

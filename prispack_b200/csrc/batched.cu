@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 
 #include "../../include/prism_solve.h"
 #include "kernels.cuh"
@@ -513,33 +514,99 @@ void launch_bt_unpack(cudaStream_t st, const Handle& h, uint32_t n, uint32_t k, 
     PRISM_LAUNCHED();
 }
 
+// A block sweep with its output marked where the kernel needs that.
+void run_block_sweep(const Handle& h, cudaStream_t st, const DevSweep& s, uint32_t k, const double* in, double* out) {
+    if (!s.self_filling()) launch_bt_fill(st, h, (uint64_t)s.n * k, out);
+    launch_bt_sweep(h, st, s, k, in, out);
+}
+
+bool BlockSweep::keeps_level() const {
+    for (Choice c : choice)
+        if (c == LEVEL) return true;
+    return false;
+}
+
+// Which layout a block of k columns takes, timed on zeros in `in` (after a warm-up, the best of two).
+// Level order is left out where its wavefronts alone, 2 us each (measured: 2.2 to 4.5), take longer
+// than the dataflow sweep, or where it came out far behind with another number of columns (its
+// time falls by up to 2.1 times from 32 columns to 33 and more, the dataflow sweep's grows with
+// them).  upload_level: the level-order copy, where the vector sweep is not one.
+void choose_block_sweep(Handle& h, BlockSweep& B, const DevSweep& tuned, uint32_t k, uint32_t width, const double* in,
+                        double* out, const std::function<void(DevSweep&)>& upload_level) {
+    const DevSweep& f = B.flow[width];
+    if (!f.n || f.layout != LAYOUT_FLOW) {  // empty, or in level order already: no slabs that fit
+        B.choice[k] = BlockSweep::FLOW;
+        return;
+    }
+    cudaEvent_t e[2] = {};
+    for (cudaEvent_t& x : e) PRISM_CUDA(cudaEventCreate(&x));
+    auto time = [&](const DevSweep& s, int runs) {
+        float best = 0.f;
+        for (int it = 0; it <= runs; ++it) {
+            PRISM_CUDA(cudaEventRecord(e[0], h.stream));
+            run_block_sweep(h, h.stream, s, k, in, out);
+            PRISM_CUDA(cudaEventRecord(e[1], h.stream));
+            PRISM_CUDA(cudaEventSynchronize(e[1]));
+            float ms = 0.f;
+            PRISM_CUDA(cudaEventElapsedTime(&ms, e[0], e[1]));
+            if (it == 1 || (it > 1 && ms < best)) best = ms;
+        }
+        return best;
+    };
+    constexpr float kWaveMs = 0.002f;
+    BlockSweep::Choice choice = BlockSweep::FLOW;
+    float flow_ms = time(f, 1);
+    if (flow_ms > (float)f.num_levels * kWaveMs && flow_ms > 0.4f * B.level_ms) {
+        const bool own = tuned.layout != LAYOUT_LEVEL;
+        if (own && !B.level.n) {
+            DevSweep d;
+            upload_level(d);
+            B.level = std::move(d);
+        }
+        B.level_ms = time(own ? B.level : tuned, 2);
+        flow_ms = std::min(flow_ms, time(f, 1));
+        if (B.level_ms < flow_ms) choice = own ? BlockSweep::LEVEL : BlockSweep::TUNED;
+    }
+    for (cudaEvent_t x : e) cudaEventDestroy(x);
+    h.check_status();
+    B.choice[k] = choice;
+    if (!B.keeps_level()) B.level.release();
+}
+
 // ============================================================================
 // Triangular preconditioner on a block: copies of the sweeps for block_columns(k)
 // columns a CTA, uploaded on first use
 // ============================================================================
+const DevSweep& TriangularPrecond::block_copy(cudaStream_t st, uint32_t k, bool lower, double* out) {
+    const uint32_t n = h_.A.n, cols = block_columns(k, n), w = block_width_index(cols);
+    BlockSweep& B = lower ? lower_bk_ : upper_bk_;
+    const DevSweep& tuned = lower ? lower_ : upper_;
+    if (B.flow[w].n != n) {
+        DevSweep d;
+        if (f_->fp32) d.upload_block(lower ? f_->lower32 : f_->upper32, h_.info, cols, h_.stream);
+        else d.upload_block(lower ? f_->lower64 : f_->upper64, h_.info, cols, h_.stream);
+        refresh_block_copy(d, w, lower);  // after a device refactorisation: its values
+        B.flow[w] = std::move(d);
+    }
+    B.flow[w].block_workspace(k, st);
+    if (B.choice[k] == BlockSweep::UNTIMED) {
+        PRISM_CUDA(cudaMemsetAsync(tmpk_.get(), 0, (size_t)n * k * sizeof(double), st));
+        choose_block_sweep(h_, B, tuned, k, w, tmpk_.get(), out, [&](DevSweep& d) {
+            if (f_->fp32) d.upload(lower ? f_->lower32 : f_->upper32, h_.info, LAYOUT_LEVEL, h_.stream);
+            else d.upload(lower ? f_->lower64 : f_->upper64, h_.info, LAYOUT_LEVEL, h_.stream);
+            refresh_block_copy(d, kBlockWidths, lower);
+        });
+    }
+    return B.of(k, w, tuned);
+}
+
 void TriangularPrecond::apply_batched(cudaStream_t st, uint32_t k, const double* in, double* out) {
-    const uint32_t n = h_.A.n;
-    const uint32_t cols = block_columns(k, n), w = block_width_index(cols);
-    auto copy = [&](DevSweep& mine, bool lower) -> const DevSweep& {
-        if (mine.n != n) {
-            DevSweep d;
-            if (f_->fp32) d.upload_block(lower ? f_->lower32 : f_->upper32, h_.info, cols, h_.stream);
-            else d.upload_block(lower ? f_->lower64 : f_->upper64, h_.info, cols, h_.stream);
-            refresh_block_copy(d, w, lower);  // after a device refactorisation: its values
-            mine = std::move(d);
-        }
-        mine.block_workspace(k, st);
-        return mine;
-    };
-    const DevSweep& lo = copy(lower_bk_[w], true);
-    const DevSweep& up = copy(upper_bk_[w], false);
-    const size_t nk = (size_t)n * k;
+    const size_t nk = (size_t)h_.A.n * k;
     if (tmpk_.size() < nk) tmpk_.alloc(nk);
-    if (!lo.self_filling()) launch_bt_fill(st, h_, nk, tmpk_.get());
-    if (in != out && !up.self_filling()) launch_bt_fill(st, h_, nk, out);
-    launch_bt_sweep(h_, st, lo, k, in, tmpk_.get());
-    if (in == out && !up.self_filling()) launch_bt_fill(st, h_, nk, out);
-    launch_bt_sweep(h_, st, up, k, tmpk_.get(), out);
+    const DevSweep& lo = block_copy(st, k, true, out);
+    const DevSweep& up = block_copy(st, k, false, out);
+    run_block_sweep(h_, st, lo, k, in, tmpk_.get());
+    run_block_sweep(h_, st, up, k, tmpk_.get(), out);
 }
 
 // ============================================================================

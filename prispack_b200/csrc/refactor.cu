@@ -391,7 +391,7 @@ struct RefactorState {
     DevBuf<int> status;       // [status, first bad column]
     DevBuf<unsigned> bad;     // first out-of-range map entry: [coefficients, diagonals]
     SweepValueMap lower, upper;
-    SweepValueMap lower_bk[kBlockWidths], upper_bk[kBlockWidths];  // of the copies for the block sweeps
+    SweepValueMap lower_bk[kBlockWidths + 1], upper_bk[kBlockWidths + 1];  // of the copies for blocks (the last: level order)
     bool refactored = false;  // the device factor differs from the host one
 };
 void refactor_release(RefactorState* r) { delete r; }
@@ -699,9 +699,11 @@ void TriangularPrecond::refactor() {
         apply_map<double>(h_, st, lower_, R.lower, R.lt64.get(), lt_n, D, ic, R.bad.get());
         apply_map<double>(h_, st, upper_, R.upper, R.lt64.get(), lt_n, D, ic, R.bad.get());
     }
-    for (uint32_t w = 0; w < kBlockWidths; ++w) {
-        if (lower_bk_[w].n) refresh_block_copy(lower_bk_[w], R.lower_bk[w], true);
-        if (upper_bk_[w].n) refresh_block_copy(upper_bk_[w], R.upper_bk[w], false);
+    for (uint32_t c = 0; c <= kBlockWidths; ++c) {
+        DevSweep& lo = c < kBlockWidths ? lower_bk_.flow[c] : lower_bk_.level;
+        DevSweep& up = c < kBlockWidths ? upper_bk_.flow[c] : upper_bk_.level;
+        if (lo.n) refresh_block_copy(lo, R.lower_bk[c], true);
+        if (up.n) refresh_block_copy(up, R.upper_bk[c], false);
     }
     check_maps(R, st, "the sweeps");
     R.refactored = true;
@@ -729,11 +731,11 @@ void TriangularPrecond::refresh_block_copy(DevSweep& d, SweepValueMap& M, bool l
 
 // A copy for the block sweeps uploaded from the host factor: nothing to do until the device has
 // refactored it.
-void TriangularPrecond::refresh_block_copy(DevSweep& d, uint32_t width, bool lower) {
+void TriangularPrecond::refresh_block_copy(DevSweep& d, uint32_t copy, bool lower) {
     if (!rf_ || !rf_->refactored) return;
     RefactorState& R = *rf_;
     PRISM_CUDA(cudaMemsetAsync(R.bad.get(), 0, 2 * sizeof(unsigned), h_.stream));
-    refresh_block_copy(d, lower ? R.lower_bk[width] : R.upper_bk[width], lower);
+    refresh_block_copy(d, lower ? R.lower_bk[copy] : R.upper_bk[copy], lower);
     check_maps(R, h_.stream, "a block copy");
 }
 

@@ -140,6 +140,24 @@ struct DevSweep {
     float tuned_ms = 0.f;          // time of the chosen kernel at setup (0: not tuned)
 };
 
+// A sweep for blocks of columns: a dataflow copy for each number of columns a CTA takes
+// (block_columns), and level order for the blocks that are faster on it.  Which of the two a block
+// of k columns takes is timed when the first one of k columns comes (choose_block_sweep): one
+// wavefront after another over the whole chip suits few and wide ones whose rows read far and
+// wide, slabs the others, and more columns cost the slabs more (random pattern of 20,000 rows,
+// 8 / 64 columns, us an IC apply: 202 / 467 dataflow, 174 / 141 level order; 512^2: 1,286 / 2,804
+// and 43,126 / 24,431).
+struct BlockSweep {
+    enum Choice : uint8_t { UNTIMED = 0, FLOW, LEVEL, TUNED };  // TUNED: the vector sweep's own, in level order
+    DevSweep flow[kBlockWidths], level;
+    Choice choice[65] = {};        // by k
+    float level_ms = 0.f;          // of the last level-order sweep timed
+    bool keeps_level() const;
+    const DevSweep& of(uint32_t k, uint32_t width, const DevSweep& tuned) const {
+        return choice[k] == TUNED ? tuned : (choice[k] == LEVEL ? level : flow[width]);
+    }
+};
+
 class Precond {
   public:
     Precond();
@@ -215,12 +233,13 @@ class TriangularPrecond : public Precond {
   private:
     int export_refactored(int which, uint32_t* n, uint64_t* nnz, uint32_t* rowptr, uint32_t* col, double* val,
                           double* diag) const;
+    const DevSweep& block_copy(cudaStream_t st, uint32_t k, bool lower, double* out);
     void refresh_block_copy(DevSweep& d, SweepValueMap& map, bool lower);
-    void refresh_block_copy(DevSweep& d, uint32_t width, bool lower);
+    void refresh_block_copy(DevSweep& d, uint32_t copy, bool lower);
     Handle& h_;
     std::shared_ptr<const HostFactor> f_;
     DevSweep lower_, upper_;
-    DevSweep lower_bk_[kBlockWidths], upper_bk_[kBlockWidths];  // copies for the block sweeps, by block_columns
+    BlockSweep lower_bk_, upper_bk_;
     DevBuf<double> tmp_, tmpk_;
     std::unique_ptr<RefactorState, void (*)(RefactorState*)> rf_{nullptr, refactor_release};
 };
@@ -272,13 +291,14 @@ class AmsedPrecond : public Precond {
     void c_solve(cudaStream_t st, int level, double* x);
     // block apply (built on first use for a given k)
     struct BlockLevel {
-        DevSweep lower[kBlockWidths], upper[kBlockWidths];  // the level's sweeps for blocks, by block_columns
+        BlockSweep lower, upper;          // the level's sweeps for blocks
         uint32_t rpad = 0, ldw = 0;       // rank rounded up to 16, rows rounded up to 16
         DevBuf<uint16_t> Wc, Wr;          // BF16 W: column-major rpad x ldw, row-major ldw x rpad
         DevBuf<float> H32;                // [rpad], zero padded
         DevBuf<double> xc, tmp, tmp2;     // nrem x k, nb x k, nb x k
     };
     void prepare_block(uint32_t k);
+    void block_buffers(uint32_t k);
     void block_solve_k(cudaStream_t st, int level, uint32_t k, const double* in, double* out);
     void c_solve_k(cudaStream_t st, int level, uint32_t k, double* x);
     void lowrank_k(cudaStream_t st, int level, uint32_t k, const double* xc, double* y);

@@ -308,6 +308,7 @@ void AmsedPrecond::block_buffers(uint32_t k) {
     cudaStream_t st = h_.stream;
     tensor_lowrank_ = a_->fp32;
     const bool first = bk_ == 0;
+    bk_ = 0;  // until all are there
     size_t part64 = 1, part32 = 1, t64 = 1, t32 = 1;
     uint32_t max_nfac = 1;
     for (uint32_t l = 0; l < nlev_; ++l) {

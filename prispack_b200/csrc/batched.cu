@@ -439,8 +439,7 @@ static BatchWork& batch_work(Handle& h, uint32_t k) {
     const uint32_t n = h.A.n;
     if (!h.batch || h.batch->n != n || h.batch->k < k) {
         h.batch.reset();
-        auto* w = new BatchWork();
-        h.batch = std::unique_ptr<BatchWork, void (*)(BatchWork*)>(w, batch_release);
+        std::unique_ptr<BatchWork, void (*)(BatchWork*)> w(new BatchWork(), batch_release);
         w->n = n;
         w->k = k;
         const size_t nk = (size_t)n * k;
@@ -452,6 +451,7 @@ static BatchWork& batch_work(Handle& h, uint32_t k) {
         w->active.alloc(kBK);
         PRISM_CUDA(cudaMallocHost(&w->pinned, kBScalars * kBK * sizeof(double)));
         PRISM_CUDA(cudaMallocHost(&w->pinned_active, kBK * sizeof(int)));
+        h.batch = std::move(w);  // whole
     }
     return *h.batch;
 }

@@ -569,7 +569,7 @@ int32_t prism_spmv(prism_handle h, const double* x, double* y) {
     return guarded([&]() -> int {
         DeviceGuard g(h->info.device);
         const uint32_t n = h->A.n;
-        if (h->xb.size() < n) { h->xb.alloc(n); h->bb.alloc(n); }
+        if (h->bb.size() < n) { h->xb.alloc(n); h->bb.alloc(n); }
         PRISM_CUDA(cudaMemcpyAsync(h->xb.get(), x, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         h->spmv(h->xb.get(), h->bb.get());
         PRISM_CUDA(cudaMemcpyAsync(y, h->bb.get(), n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -924,7 +924,7 @@ int32_t prism_apply(prism_handle h, const double* in, double* out) {
     return guarded([&]() -> int {
         DeviceGuard g(h->info.device);
         const uint32_t n = h->A.n;
-        if (h->xb.size() < n) { h->xb.alloc(n); h->bb.alloc(n); }
+        if (h->bb.size() < n) { h->xb.alloc(n); h->bb.alloc(n); }
         PRISM_CUDA(cudaMemcpyAsync(h->bb.get(), in, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         h->P->apply(h->stream, h->bb.get(), h->xb.get());
         PRISM_CUDA(cudaMemcpyAsync(out, h->xb.get(), n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -996,7 +996,7 @@ int32_t prism_solve(prism_handle h, const prism_solve_opts* opts, const double* 
     return guarded([&]() -> int {
         DeviceGuard g(h->info.device);
         const uint32_t n = h->A.n;
-        if (h->xb.size() < n) { h->xb.alloc(n); h->bb.alloc(n); }
+        if (h->bb.size() < n) { h->xb.alloc(n); h->bb.alloc(n); }
         PRISM_CUDA(cudaMemcpyAsync(h->bb.get(), b, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         PRISM_CUDA(cudaMemcpyAsync(h->xb.get(), x, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         const double* xref = nullptr;

@@ -53,6 +53,7 @@ class DevBuf {
         if (count == 0) return;
         cudaError_t e = cudaMalloc(&p_, count * sizeof(T));
         if (e != cudaSuccess) {
+            cudaGetLastError();  // reported here; not to the next launch
             p_ = nullptr;
             throw Error(8, std::string("cudaMalloc(") + std::to_string(count * sizeof(T)) + " B): " + cudaGetErrorString(e));
         }

@@ -334,6 +334,7 @@ struct GmresWork {
     void ensure(uint32_t n_, uint32_t ld_, int grid_, cudaStream_t s) {
         if (n_ == n && ld_ == ld && grid_ <= grid) return;
         graph.reset();
+        n = 0;  // until all are there
         H.alloc((size_t)ld_ * (ld_ - 1));
         cs.alloc(ld_);
         sn.alloc(ld_);

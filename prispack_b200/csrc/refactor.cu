@@ -558,8 +558,8 @@ void TriangularPrecond::refactor() {
         }
     }
     if (!rf_) {
-        rf_.reset(new RefactorState());
-        RefactorState& R = *rf_;
+        std::unique_ptr<RefactorState, void (*)(RefactorState*)> built(new RefactorState(), refactor_release);
+        RefactorState& R = *built;
         // a diagonal factor has no updates and, ILDLT, no entries
         auto put = [&](DevBuf<uint32_t>& d, const std::vector<uint32_t>& v) {
             d.alloc(std::max<size_t>(v.size(), 1));
@@ -630,6 +630,7 @@ void TriangularPrecond::refactor() {
             build_map<double>(upper_, F.upper64, iup, R.upper, st);
         }
         PRISM_CUDA(cudaStreamSynchronize(st));
+        rf_ = std::move(built);  // whole
     }
     RefactorState& R = *rf_;
     RfArgs a;

@@ -197,8 +197,7 @@ void segmented_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t nseg, co
                         throw Error(PRISM_ERR_ARG, "row " + std::to_string(i) + " couples system " +
                                                        std::to_string(s) + " to another one");
         h.seg.reset();
-        auto* w = new SegWork();
-        h.seg = std::unique_ptr<SegWork, void (*)(SegWork*)>(w, seg_release);
+        std::unique_ptr<SegWork, void (*)(SegWork*)> w(new SegWork(), seg_release);
         w->seg.assign(seg_ptr, seg_ptr + nseg + 1);
         std::vector<uint32_t> lo, of, first;
         for (uint32_t s = 0; s < nseg; ++s) {
@@ -221,6 +220,7 @@ void segmented_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t nseg, co
         w->sc.alloc((size_t)kSegScalars * nseg);
         w->active.alloc(nseg);
         w->host.assign((size_t)kSegScalars * nseg, 0.0);
+        h.seg = std::move(w);  // whole
     }
     SegWork& w = *h.seg;
     h.ensure_workspace();

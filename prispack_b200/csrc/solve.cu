@@ -431,7 +431,7 @@ Handle::~Handle() {
 
 void Handle::ensure_workspace() {
     const uint32_t n = A.n;
-    if (r.size() < n) {
+    if (y.size() < n) {  // the last one: all are there
         r.alloc(n); w.alloc(n); d.alloc(n); v.alloc(n); y.alloc(n);
     }
 }
@@ -856,15 +856,21 @@ template void stream_sweep_run<float>(int, const Sweep<float>&, bool, uint32_t, 
 template <typename Low>
 void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pair) {
     const int mode = h.info.sweep_kernel;
-    const bool a32 = d.acc32 = acc32 && std::is_same<Low, float>::value;
+    const bool a32 = acc32 && std::is_same<Low, float>::value;
     // Pairing keeps the arithmetic's precision class only where the derived coefficients are
     // stored in the arithmetic's own type: double values (FP64) or float values with float
     // arithmetic; float values with double arithmetic (<float,double>) stay unpaired.
     const bool pp = pair && h.info.stream_pair != 0 && (a32 || std::is_same<Low, double>::value);
     const bool only_paired = pp && h.info.stream_pair == 2;  // paired where it fits
     const bool any = mode == 0 && !a32 && !only_paired;      // every layout is a candidate
+    auto untimed = [&](int layout) {
+        DevSweep t;
+        t.acc32 = a32;
+        t.upload(s, h.info, layout, h.stream);
+        d = std::move(t);
+    };
     if (s.n == 0 || (mode != 0 && mode != 3 && !a32 && !only_paired)) {
-        d.upload(s, h.info, s.n != 0 && mode == 2 ? LAYOUT_SLAB : LAYOUT_LEVEL, h.stream);
+        untimed(s.n != 0 && mode == 2 ? LAYOUT_SLAB : LAYOUT_LEVEL);
         return;
     }
     struct Paired {
@@ -979,7 +985,7 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
         streamed(p.s, &p.m, size);
     }
     if (best == kNever) {  // nothing fitted (streamed layouts only): level order, double arithmetic
-        d.upload(s, h.info, LAYOUT_LEVEL, h.stream);
+        untimed(LAYOUT_LEVEL);
         return;
     }
     d = std::move(kept);

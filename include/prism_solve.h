@@ -439,8 +439,8 @@ int32_t prism_solve(prism_handle h, const prism_solve_opts* opts, const double* 
  * factor: with the values the factor was built from, the result is the host
  * factor bit for bit.  The new values go into every device layout of the
  * preconditioner's sweeps.  PRISM_ERR_NOT_SPD / PRISM_ERR_ZERO_PIVOT as the
- * host factorisation reports them; PRISM_ERR_UNSUPPORTED for ILUT, AMSED and
- * GMSLR.
+ * host factorisation reports them, the factor and its sweeps then staying as
+ * they were; PRISM_ERR_UNSUPPORTED for ILUT, AMSED and GMSLR.
  *
  * prism_adjoint_solve*: the backward pass of x = A^{-1} b for a scalar loss L
  * with g = dL/dx:  lambda = A^{-T} g  (= dL/db), solved with the handle's

@@ -386,8 +386,10 @@ struct RefactorState {
     DevBuf<uint64_t> uo, so;  // per column: its first update entry; its first chunk's segments
     DevBuf<uint16_t> place, seg;  // as RfArgs
     uint32_t smax = 0;
-    DevBuf<float> lt32;
-    DevBuf<double> lt64, D;
+    // the factor values and pivots the sweeps hold, and those a refactorisation writes: swapped
+    // where it succeeds, so that one that fails leaves the factor as it was
+    DevBuf<float> lt32, lt32_new;
+    DevBuf<double> lt64, lt64_new, D, D_new;
     DevBuf<int> status;       // [status, first bad column]
     DevBuf<unsigned> bad;     // first out-of-range map entry: [coefficients, diagonals]
     SweepValueMap lower, upper;
@@ -615,9 +617,10 @@ void TriangularPrecond::refactor() {
         R.place.alloc(std::max<uint64_t>(uo[P.n], 1));
         R.seg.alloc(std::max<uint64_t>(so[P.n], 1));
         const size_t nnz = std::max<size_t>(F.f0.col.size(), 1);
-        if (F.fp32) R.lt32.alloc(nnz);
-        else R.lt64.alloc(nnz);
+        if (F.fp32) R.lt32.alloc(nnz), R.lt32_new.alloc(nnz);
+        else R.lt64.alloc(nnz), R.lt64_new.alloc(nnz);
         R.D.alloc(std::max<uint32_t>(P.n, 1));
+        R.D_new.alloc(std::max<uint32_t>(P.n, 1));
         R.status.alloc(2);
         R.bad.alloc(2);
         Sweep<double> ilo, iup;
@@ -676,9 +679,9 @@ void TriangularPrecond::refactor() {
     if (occ < 1) throw Error(PRISM_ERR_UNSUPPORTED, "the refactorisation kernel does not fit on an SM");
     const uint64_t want = ((uint64_t)P.n + kRfWarps - 1) / kRfWarps;
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)h_.info.sms * occ));
-    void* lt = F.fp32 ? (void*)R.lt32.get() : (void*)R.lt64.get();
-    double* D = R.D.get();
-    void* args[] = {&a, &lt, &D};
+    void* lt = F.fp32 ? (void*)R.lt32_new.get() : (void*)R.lt64_new.get();
+    double* D_new = R.D_new.get();
+    void* args[] = {&a, &lt, &D_new};
     PRISM_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, st));
     PRISM_LAUNCHED();
     int hs[2] = {0, 0};
@@ -689,6 +692,10 @@ void TriangularPrecond::refactor() {
     if (hs[0] == PRISM_ERR_ZERO_PIVOT)
         throw Error(PRISM_ERR_ZERO_PIVOT, "refactorisation: zero pivot in column " + std::to_string(hs[1]));
     if (hs[0] != 0) throw Error(hs[0], "refactorisation: a dependency wait ran out in column " + std::to_string(hs[1]));
+    std::swap(R.lt32, R.lt32_new);
+    std::swap(R.lt64, R.lt64_new);
+    std::swap(R.D, R.D_new);
+    const double* D = R.D.get();
     // the new values into every device layout of the two sweeps
     const bool ic = F.kind == 1;
     const uint64_t lt_n = F.f0.col.size();

@@ -62,3 +62,30 @@ def test_copies_are_kept():
     apply(), refactor(), apply()
     # the two alone take about 4 ms here and the layout of both sweeps about 100 ms
     assert best(refactor, apply) <= 4 * (best(refactor) + best(apply))
+
+
+@pytest.mark.parametrize("kind,precision", [(P.PRECOND_IC, P.PRISM_FP64), (P.PRECOND_ILDLT, P.PRISM_FP32)])
+def test_a_failed_refactorisation_leaves_the_factor(kind, precision):
+    """The vector sweeps, the factor as it is read back and copies for blocks uploaded afterwards
+    all hold the last factor that was completed."""
+    A = P.CSRMatrix.laplacian(24, 20, 3)
+    S = P.DeviceSystem(A)
+    S.set_precond(kind, tol=1e-3, precision=precision)
+    S.update_values(new_values(A, seed=30))
+    S.refactor()
+    v = np.random.default_rng(1).standard_normal(A.n)
+    before, factor = S.apply(v), S.precond_factor(0)
+    rows = np.repeat(np.arange(A.n), np.diff(A.rowptr))
+    bad = A.val.copy()
+    # a pivot with no square root after most columns are done, or nothing to divide the first by
+    at, value = (A.n - 40, -1.0) if kind == P.PRECOND_IC else (0, 0.0)
+    bad[(rows == at) & (A.col == at)] = value
+    S.update_values(bad)
+    with pytest.raises(P.PrismError) as e:
+        S.refactor()
+    assert e.value.status == (4 if kind == P.PRECOND_IC else 3)
+    assert np.array_equal(S.apply(v), before)
+    for got, want in zip(S.precond_factor(0), factor):
+        if want is not None:
+            assert np.array_equal(got, want)
+    blocks_match(S, (3, 30), 7)

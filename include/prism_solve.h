@@ -393,7 +393,8 @@ int32_t prism_apply(prism_handle h, const double* in, double* out);
  * 2: mark out_d pending only.  prism_precond_sweep_info reports the sweep's
  * rows, stored non-zeros, bytes per stored value, wavefront count and the
  * kernel the setup-time autotuner kept (1: level-ordered grid-wide sweep,
- * 2: slab-blocked sweep with shared-memory dependencies). */
+ * 2: slab-blocked sweep with shared-memory dependencies, 3: dataflow slabs,
+ * 4: streamed rounds). */
 int32_t prism_precond_sweep_device(prism_handle h, int32_t sweep, const double* in_d, double* out_d,
                                    int32_t prepare);
 int32_t prism_precond_sweep_info(prism_handle h, int32_t sweep, uint32_t* n, uint64_t* nnz,

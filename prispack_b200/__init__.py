@@ -760,7 +760,7 @@ class DeviceSystem:
         _check(self.lib.prism_precond_sweep_info(self.h, sweep, C.byref(n), C.byref(nnz), C.byref(vb), C.byref(lv),
                                                  C.byref(kk)))
         return {"n": n.value, "nnz": nnz.value, "value_bytes": vb.value, "levels": lv.value,
-                "kernel": {1: "level-order", 2: "slab", 3: "stream"}.get(kk.value, "?")}
+                "kernel": {1: "level-order", 2: "slab", 3: "stream", 4: "rounds"}.get(kk.value, "?")}
 
     def sweep_order(self, sweep: int) -> SweepOrder:
         """Summation order of one of the preconditioner's sweeps when it runs the streamed kernel

@@ -529,7 +529,7 @@ bool AmsedPrecond::sweep_info(int sweep, uint32_t* n, uint64_t* nnz, uint32_t* v
     if (nnz) *nnz = s.entries();
     if (vbytes) *vbytes = s.fp32 ? 4 : 8;
     if (levels) *levels = s.num_levels;
-    if (kernel) *kernel = s.streamed() ? 3 : (s.layout == LAYOUT_SLAB ? 2 : 1);
+    if (kernel) *kernel = s.kernel_id();
     return true;
 }
 

@@ -373,6 +373,7 @@ int selftest_wait_timeout(int device, unsigned long long wait_ns, int* device_st
 void init_device_info(DeviceInfo& info, int device) {
     info.device = device;
     PRISM_CUDA(cudaDeviceGetAttribute(&info.sms, cudaDevAttrMultiProcessorCount, device));
+    info.co_resident = info.sms;
     int occ = 0, occ2 = 0;
     PRISM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sweep<double, OP_DIV>, kBlock, 0));
     PRISM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_sweep<float, OP_DIV>, kBlock, 0));
@@ -386,7 +387,7 @@ void init_device_info(DeviceInfo& info, int device) {
     PRISM_CUDA(cudaDeviceGetAttribute(&info.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     if (const char* e = std::getenv("PRISM_SWEEP_KERNEL")) {
         const std::string k(e);
-        info.sweep_kernel = k == "global" ? 1 : (k == "slab" ? 2 : (k == "stream" ? 3 : 0));
+        info.sweep_kernel = k == "global" ? 1 : (k == "slab" ? 2 : (k == "stream" ? 3 : (k == "rounds" ? 4 : 0)));
     }
     if (const char* e = std::getenv("PRISM_SLAB_MIN_ROWS")) info.slab_min_rows = (uint32_t)std::atoi(e);
     if (const char* e = std::getenv("PRISM_SLAB_MAX_ROWS")) info.slab_max_rows = (uint32_t)std::atoi(e);
@@ -548,6 +549,7 @@ StreamPlan plan_stream(const Sweep<Low>& s0, const DeviceInfo& info, bool acc32)
     if (nn == 0) return P;
     const uint32_t ctas_req = stream_slab_count(nn, (uint32_t)info.sms, info.stream_min_rows);
     const std::vector<uint32_t> start = slab_ranges<Low>(s0, ctas_req);
+    if (start.size() - 1 > (size_t)info.co_resident) return P;  // one co-resident CTA a slab: too many independent blocks
     const uint64_t smem = (uint64_t)info.max_smem_optin;
     StreamLayout& L = P.L;
     const bool a32 = acc32 && std::is_same<Low, float>::value;
@@ -869,7 +871,7 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
         t.upload(s, h.info, layout, h.stream);
         d = std::move(t);
     };
-    if (s.n == 0 || (mode != 0 && mode != 3 && !a32 && !only_paired)) {
+    if (s.n == 0 || ((mode == 1 || mode == 2) && !a32 && !only_paired)) {
         untimed(s.n != 0 && mode == 2 ? LAYOUT_SLAB : LAYOUT_LEVEL);
         return;
     }
@@ -923,8 +925,9 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
         t.acc32 = a32;
         if (t.upload(s, h.info, layout, h.stream)) time(std::move(t));
     };
+    const bool rounds = mode == 4;
     // small sweeps: the smallest size (64^2: 8% faster than the others)
-    const bool climbs = !h.info.flow_rows && s.n > 32 * kFlowSlabRows[0];
+    const bool climbs = !rounds && !h.info.flow_rows && s.n > 32 * kFlowSlabRows[0];
     const uint32_t only_rows = h.info.flow_rows ? h.info.flow_rows : kFlowSlabRows[0];
     // the unpaired layouts that are needed in any case: on the host while the one before is timed
     int size = 1;
@@ -945,7 +948,8 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
         };
         bool first = true;
         auto flow = [&](uint32_t rows) {
-            StreamPlan P = rows == ahead_rows ? ahead.get() : plan_flow<Low>(sw, h.info, a32, rows);
+            StreamPlan P;
+            if (!rounds) P = rows == ahead_rows ? ahead.get() : plan_flow<Low>(sw, h.info, a32, rows);
             ahead_rows = 0;
             if (first && !pm && climbs) lay_ahead(kFlowSlabRows[at - 1]);
             if (!P.ok && first) P = plan_stream<Low>(sw, h.info, a32);
@@ -974,7 +978,7 @@ void tune_sweep(Handle& h, DevSweep& d, const Sweep<Low>& s, bool acc32, bool pa
         }
         return at;
     };
-    if (!only_paired) lay_ahead(climbs ? kFlowSlabRows[size] : only_rows);
+    if (!only_paired && !rounds) lay_ahead(climbs ? kFlowSlabRows[size] : only_rows);
     if (any) {
         plain(LAYOUT_LEVEL);
         plain(LAYOUT_SLAB);
@@ -1032,7 +1036,7 @@ bool TriangularPrecond::run_sweep(cudaStream_t st, int sweep, const double* in, 
 bool TriangularPrecond::sweep_info(int sweep, uint32_t* n, uint64_t* nnz, uint32_t* vbytes, uint32_t* levels,
                                    uint32_t* kernel) const {
     const DevSweep& s = sweep == 0 ? lower_ : upper_;
-    if (kernel) *kernel = s.streamed() ? 3 : (s.layout == LAYOUT_SLAB ? 2 : 1);
+    if (kernel) *kernel = s.kernel_id();
     if (n) *n = s.n;
     if (nnz) *nnz = s.entries();
     if (vbytes) *vbytes = s.fp32 ? 4 : 8;

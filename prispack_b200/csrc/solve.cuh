@@ -18,10 +18,11 @@ namespace prism {
 // Per-device launch geometry, looked up once per handle.
 struct DeviceInfo {
     int device = 0;
-    int sms = 148;
+    int sms = 148;                 // CTAs of a streamed sweep
+    int co_resident = 148;         // CTAs of a whole SM that run at the same time
     int sweep_blocks_per_sm = 1;   // co-resident k_sweep blocks (cooperative launch bound)
     int max_smem_optin = 0;        // bytes of dynamic shared memory one block may opt into
-    int sweep_kernel = 0;          // 0: autotune per sweep, 1: global level order, 2: slab-blocked, 3: streamed (dataflow or rounds)
+    int sweep_kernel = 0;          // 0: autotune per sweep, 1: global level order, 2: slab-blocked, 3: dataflow (rounds where no slab fits), 4: rounds
     uint32_t slab_min_rows = 2048; // smallest slab (small systems use fewer CTAs)
     uint32_t slab_max_rows = 1u << 30;  // largest slab (default: what shared memory holds)
     uint32_t stream_min_rows = 1024;    // smallest streamed slab (small systems use fewer CTAs)
@@ -128,6 +129,10 @@ struct DevSweep {
     template <typename Low>
     void upload_block(const Sweep<Low>& s, const DeviceInfo& info, uint32_t cols, cudaStream_t st);
     void block_workspace(uint32_t k, cudaStream_t st);  // exchange entries for k columns
+    // as prism_precond_sweep_info reports it
+    uint32_t kernel_id() const {
+        return layout == LAYOUT_FLOW ? 3 : (layout == LAYOUT_STREAM ? 4 : (layout == LAYOUT_SLAB ? 2 : 1));
+    }
     bool streamed() const { return layout == LAYOUT_STREAM || layout == LAYOUT_FLOW; }
     // the streamed layouts mark their own output pending or need no mark; the others need launch_fill first
     bool self_filling() const { return streamed(); }

@@ -142,6 +142,11 @@ uint64_t prism_kernel_launch_count(void);
  * then runs a valid sweep to show the context is still usable.  No reference
  * counterpart (the reference has no device-side waits). */
 int32_t prism_selftest_wait_timeout(int32_t device, uint64_t wait_ns, int32_t* device_status);
+/* The same of the dataflow sweep (cols = 0: one vector; 1, 2 or 4: that many
+ * columns of a block a CTA): a slab waits for a value that the slab before it
+ * does not publish; every CTA leaves, and the next sweep on the same buffers
+ * is checked against the host replay of its layout. */
+int32_t prism_selftest_flow_timeout(int32_t device, int32_t cols, uint64_t wait_ns, int32_t* device_status);
 
 /* Host self test of the streamed round layout of the triangular sweep kernel:
  * builds the sweep of the gather-form CSR (row r lists its dependencies and

@@ -74,6 +74,7 @@ _SIGS = {
     "prism_last_error": (C.c_char_p, []),
     "prism_version": (C.c_int32, []),
     "prism_kernel_launch_count": (C.c_uint64, []),
+    "prism_selftest_flow_timeout": (C.c_int32, [C.c_int32, C.c_int32, C.c_uint64, C.POINTER(C.c_int32)]),
     "prism_selftest_wait_timeout": (C.c_int32, [C.c_int32, C.c_uint64, C.POINTER(C.c_int32)]),
     "prism_lowrank_block_run": (C.c_int32, [C.c_int32, C.c_uint32, C.c_uint32, C.c_uint32, _f64p, _f64p, _f64p, _f64p,
                                             C.c_int32]),
@@ -194,6 +195,14 @@ def _check(rc: int):
 
 def kernel_launch_count() -> int:
     return int(load().prism_kernel_launch_count())
+
+
+def selftest_flow_timeout(device: int = 0, cols: int = 0, wait_ns: int = 50_000_000) -> int:
+    """Bounded-wait check of the dataflow sweep (see prism_selftest_flow_timeout): the status the
+    wait raised."""
+    st = C.c_int32()
+    _check(load().prism_selftest_flow_timeout(device, cols, wait_ns, C.byref(st)))
+    return st.value
 
 
 def selftest_wait_timeout(device: int = 0, wait_ns: int = 50_000_000) -> int:

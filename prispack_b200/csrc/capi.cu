@@ -211,6 +211,19 @@ int32_t prism_selftest_wait_timeout(int32_t device, uint64_t wait_ns, int32_t* d
     });
 }
 
+int32_t prism_selftest_flow_timeout(int32_t device, int32_t cols, uint64_t wait_ns, int32_t* device_status) {
+    if (!device_status) return fail(PRISM_ERR_ARG, "null status");
+    if (cols != 0 && cols != 1 && cols != 2 && cols != 4) return fail(PRISM_ERR_ARG, "0, 1, 2 or 4 columns");
+    if (wait_ns == 0 || wait_ns > 2000000000ull) return fail(PRISM_ERR_ARG, "wait_ns must be in (0, 2 s]");
+    return guarded([&]() -> int {
+        int s = -1;
+        DeviceGuard g(device);
+        prism::selftest_flow_timeout(device, (uint32_t)cols, wait_ns, &s);
+        *device_status = s;
+        return PRISM_OK;
+    });
+}
+
 int32_t prism_selftest_flow_layout(uint32_t n, const uint32_t* rowptr, const uint32_t* col, const double* val,
                                    const double* diag, int32_t op, int32_t lower, int32_t precision,
                                    uint32_t num_slabs, uint32_t max_slots, const double* in, double* out) {

@@ -139,7 +139,7 @@ static FlowArgs flow_args(const Handle& h, const DevSweep& s, const double* in, 
     a.in = in;
     a.out = out;
     a.status = h.status.get();
-    a.wait_ns = kWaitNs;
+    a.wait_ns = h.info.wait_ns;
     a.slabs = s.fl_slabs;
     a.slots = s.str_slots;
     a.dd = s.fl_dd.get();
@@ -840,6 +840,74 @@ void stream_sweep_run(int device, const Sweep<Low>& s, bool acc32, uint32_t num_
 }
 template void stream_sweep_run<double>(int, const Sweep<double>&, bool, uint32_t, const double*, double*);
 template void stream_sweep_run<float>(int, const Sweep<float>&, bool, uint32_t, const double*, double*);
+
+// ============================================================================
+// Bounded-wait self test of the dataflow sweep: four slabs of 128 rows whose first one keeps the
+// value of its last row to itself, so the second waits for an exchange entry that is never
+// written.  The wait runs out after wait_ns, every CTA leaves, and status 6 is raised; with the
+// header put right the same layout, exchange entries and all, then sweeps to the replay's bits.
+// ============================================================================
+void selftest_flow_timeout(int device, uint32_t cols, unsigned long long wait_ns, int* device_status) {
+    Handle h;
+    init_device_info(h.info, device);
+    h.info.wait_ns = wait_ns;
+    PRISM_CUDA(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
+    h.own_stream = true;
+    h.status.alloc(1);
+    PRISM_CUDA(cudaMemsetAsync(h.status.get(), 0, sizeof(int), h.stream));
+    // row r reads rows r - 1 and r - 37
+    const uint32_t n = 512, slab = 128, k = std::max(cols, 1u);
+    std::vector<uint32_t> rp{0}, ci;
+    std::vector<double> val;
+    for (uint32_t r = 0; r < n; ++r) {
+        if (r >= 37) ci.push_back(r - 37), val.push_back(0.25);
+        if (r >= 1) ci.push_back(r - 1), val.push_back(-0.5);
+        rp.push_back((uint32_t)ci.size());
+    }
+    Sweep<double> s;
+    build_sweep<double>(n, rp, ci, val, nullptr, SWEEP_NONE, true, s);
+    StreamPlan P = plan_flow<double>(s, h.info, false, slab, cols);
+    if (!P.ok || P.F.slabs != n / slab) throw Error(PRISM_ERR_CUDA, "four slabs expected");
+    FlowLayout good;
+    flow_layout<double>(s, slab_ranges<double>(s, P.ctas_req), P.F.slots, good, nullptr, nullptr, P.F.entries);
+    bool found = false;
+    for (size_t i = 0; i < P.F.hdr.size(); i += 4)
+        if (P.F.hdr[i] == slab - 1) {
+            found = P.F.hdr[i + 1] != kFlowNone;
+            P.F.hdr[i + 1] = kFlowNone;
+        }
+    if (!found) throw Error(PRISM_ERR_CUDA, "a published row expected");
+    DevSweep d;
+    d.commit_stream(std::move(P), h.stream);
+    d.block_workspace(k, h.stream);
+    std::vector<double> in((size_t)n * k), got((size_t)n * k), one(n), want(n);
+    for (size_t i = 0; i < in.size(); ++i) in[i] = 1.0 + (double)(i % 11) * 0.125;
+    DevBuf<double> din(in.size()), dout(in.size());
+    din.upload(in.data(), in.size(), h.stream);
+    auto sweep = [&]() {
+        if (cols) launch_flow_block(h, h.stream, d, k, din.get(), dout.get());
+        else launch_sweep(h, h.stream, d, din.get(), dout.get());
+        h.check_status();
+    };
+    *device_status = 0;
+    try {
+        sweep();
+    } catch (const Error& e) {
+        if (e.status == PRISM_ERR_CUDA) throw;
+        *device_status = e.status;
+    }
+    d.fl_hdr.upload(good.hdr.data(), good.hdr.size(), h.stream);
+    sweep();
+    PRISM_CUDA(cudaMemcpy(got.data(), dout.get(), got.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    for (uint32_t c = 0; c < k; ++c) {
+        for (uint32_t r = 0; r < n; ++r) one[r] = in[(size_t)r * k + c];
+        const std::string why = flow_layout_replay<double>(s, good, false, one.data(), want.data());
+        if (!why.empty()) throw Error(PRISM_ERR_CUDA, "dataflow layout: " + why);
+        for (uint32_t r = 0; r < n; ++r)
+            if (got[(size_t)r * k + c] != want[r])
+                throw Error(PRISM_ERR_CUDA, "the sweep after the one that was given up differs in row " + std::to_string(r));
+    }
+}
 
 // Sweep-kernel autotuner: uploads the sweep in one device layout after another
 // (level order for k_sweep, slabs for k_sweep_slab, dataflow slabs for k_sweep_flow

@@ -19,6 +19,7 @@ namespace prism {
 struct DeviceInfo {
     int device = 0;
     int sms = 148;                 // CTAs of a streamed sweep
+    unsigned long long wait_ns = 1000000000ull;  // bound of a dataflow sweep's wait for a value
     int co_resident = 148;         // CTAs of a whole SM that run at the same time
     int sweep_blocks_per_sm = 1;   // co-resident k_sweep blocks (cooperative launch bound)
     int max_smem_optin = 0;        // bytes of dynamic shared memory one block may opt into
@@ -402,6 +403,8 @@ void lowrank_block_run(int device, uint32_t nrem, uint32_t rank, uint32_t k, con
 
 // Runs the bounded-wait self test (see solve.cu); returns the device status the wait raised.
 int selftest_wait_timeout(int device, unsigned long long wait_ns, int* device_status);
+// the same for the dataflow sweep, on one vector (cols = 0) or a block of cols columns
+void selftest_flow_timeout(int device, uint32_t cols, unsigned long long wait_ns, int* device_status);
 
 // Queries SM count and the co-resident capacity of the sweep kernel.
 void init_device_info(DeviceInfo& info, int device);

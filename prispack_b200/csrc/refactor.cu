@@ -576,7 +576,10 @@ void TriangularPrecond::refactor() {
         put(R.up_start, P.up_start);
         R.done.alloc(P.n);
         PRISM_CUDA(cudaMemsetAsync(R.done.get(), 0, (size_t)P.n * sizeof(uint32_t), st));
-        R.smax = std::max<uint32_t>(512, (P.max_col + 31) / 32 * 32);
+        // Longer columns leave one CTA an SM in any case, so their chunks take all the products a
+        // place can name (columns of 600 entries, a full factor, ms: 534 with one update a chunk,
+        // 384 now; a warp pass per update took 464).
+        R.smax = P.max_col <= 512 ? 512u : kRfPlace + 1;
         // where each column's update entries start, and the segments of its chunks (cut as RfChunk
         // cuts them); what stands there is found on the device, once
         std::vector<uint64_t> uo((size_t)P.n + 1, 0), so((size_t)P.n + 1, 0);

@@ -99,13 +99,36 @@ static __global__ void __launch_bounds__(kBlock) k_bk_sub(uint64_t count, const 
 // ---------------------------------------------------------------------------
 // Block partials of W^T X for rank columns q and block columns c: thread (g, c) with
 // g = threadIdx.x / 64 sums q = g, g + 4, ... over the block's rows (grid-stride by
-// tiles of kLrTile rows); the last block adds the partials in block order and scales by H.
-// Rows a block takes at a time, and at most one block an SM: with 64 rows a block, six blocks
-// worked on the 371 rows below the first level of a 95 x 71 grid (13 columns: 33 us).
+// tiles of kLrTile rows).  The partials are added up in two steps, each in order: the last block
+// of a group of about sqrt(blocks) adds up the group's, the last group's the groups', scaled by H.
+// Rows a block takes at a time: with 64 rows a block, six blocks worked on the 371 rows below the
+// first level of a 95 x 71 grid (13 columns: 33 us); lr_grid has the number of blocks.  One block
+// adding up all partials reads them at an SM's rate: 5,000 rows, rank 32, 64 columns 106 us with
+// 148 partials, 42 now.
 constexpr uint32_t kLrTile = 8;
+constexpr uint32_t kLrTickets = 64;  // one, and one a group (at most sqrt of four blocks an SM)
+__host__ __device__ inline uint32_t lr_group(uint32_t blocks) {
+    uint32_t g = 1;
+    while (g * g < blocks) ++g;
+    return g;
+}
+// The sums of partials first, first + step, ... (count of them), in order, to put(q, c, sum).
+template <typename Put>
+__device__ __forceinline__ void lr_sum(const double* partial, uint32_t r, uint32_t k, uint32_t first, uint32_t step,
+                                       uint32_t count, Put put) {
+    for (uint32_t e = threadIdx.x; e < r * k; e += blockDim.x) {
+        const uint32_t q = e / k, c = e - q * k;
+        const double* p = partial + ((size_t)first * r + q) * kLrMaxK + c;
+        const size_t d = (size_t)step * r * kLrMaxK;
+        double s = 0.0;
+#pragma unroll 8
+        for (uint32_t b = 0; b < count; ++b) s += __ldcg(p + b * d);
+        put(q, c, s);
+    }
+}
 static __global__ void __launch_bounds__(kBlock) k_lr_dots_f64(uint32_t nrem, uint32_t k, uint32_t r,
                                                                const double* __restrict__ W, const double* __restrict__ H,
-                                                               const double* __restrict__ X, double* __restrict__ partial,
+                                                               const double* __restrict__ X, double* partial,
                                                                unsigned* __restrict__ ticket, double* __restrict__ T) {
     const uint32_t c = threadIdx.x & 63, g = threadIdx.x >> 6;
     for (uint32_t q0 = 0; q0 < r; q0 += 32) {
@@ -133,24 +156,27 @@ static __global__ void __launch_bounds__(kBlock) k_lr_dots_f64(uint32_t nrem, ui
         }
     }
     __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    auto is_last = [&](unsigned* t, uint32_t of) {
         __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (uint32_t e = threadIdx.x; e < r * kLrMaxK; e += blockDim.x) {
-        const uint32_t q = e / kLrMaxK, cc = e % kLrMaxK;
-        if (cc >= k) continue;
-        double s = 0.0;
-#pragma unroll 4
-        for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(partial + ((size_t)b * r + q) * kLrMaxK + cc);
-        T[(size_t)q * kLrMaxK + cc] = s * H[q];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) *ticket = 0u;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            last = atomicAdd(t, 1u) == of - 1;
+            if (last) *t = 0u;
+        }
+        __syncthreads();
+        __threadfence();
+        return last;
+    };
+    const uint32_t size = lr_group(gridDim.x), groups = (gridDim.x + size - 1) / size, group = blockIdx.x / size;
+    const uint32_t first = group * size, members = min(size, gridDim.x - first);
+    if (!is_last(ticket + 1 + group, members)) return;
+    if (members > 1 && groups > 1)
+        lr_sum(partial, r, k, first, 1, members, [&](uint32_t q, uint32_t cc, double s) {
+            partial[((size_t)first * r + q) * kLrMaxK + cc] = s;
+        });
+    if (groups > 1 && !is_last(ticket, groups)) return;
+    lr_sum(partial, r, k, 0, groups > 1 ? size : 1, groups > 1 ? groups : members,
+           [&](uint32_t q, uint32_t cc, double s) { T[(size_t)q * kLrMaxK + cc] = s * H[q]; });
 }
 
 // Y[i][c] += sum_q W[q][i] T[q][c], q in order (DenseMatrix::MatVec column order, then x2 += ...)

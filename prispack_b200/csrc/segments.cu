@@ -26,7 +26,6 @@ enum SegScalar : int { SG_BB = 0, SG_RES, SG_RR, SG_WV, SG_DV, SG_DR, SG_DR2, kS
 // system adds up its partial sums in chunk order.  A block a system left 100 SMs idle on 48
 // systems of up to 25,600 rows: 35 to 56 us a kernel.
 constexpr uint32_t kSegChunk = 4096;
-constexpr int kSegBlock = 512;
 struct SegTable {
     uint32_t chunks;
     const uint32_t* lo;      // chunks + 1: chunk c is the rows [lo[c], lo[c + 1])
@@ -68,13 +67,14 @@ __device__ __forceinline__ void seg_store(double (&v)[NV], double* const (&out)[
 }
 
 // r = b - y (r may be null); bb[s] = Σ b², res[s] = Σ (b - y)²
-__global__ void __launch_bounds__(kSegBlock) k_seg_residual(const SegTable T, const double* __restrict__ b,
-                                                            const double* __restrict__ y, double* __restrict__ r,
-                                                            double* bb, double* res) {
+template <int B>
+__global__ void __launch_bounds__(B) k_seg_residual(const SegTable T, const double* __restrict__ b,
+                                                    const double* __restrict__ y, double* __restrict__ r,
+                                                    double* bb, double* res) {
     for (uint32_t c = blockIdx.x; c < T.chunks; c += gridDim.x) {
         double v[2] = {0.0, 0.0};
 #pragma unroll 4
-        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += kSegBlock) {
+        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += B) {
             const double bi = b[i], ri = bi - y[i];
             if (r) r[i] = ri;
             v[0] += bi * bi;
@@ -86,25 +86,27 @@ __global__ void __launch_bounds__(kSegBlock) k_seg_residual(const SegTable T, co
 }
 
 // out[s] = Σ a b over the system's rows
-__global__ void __launch_bounds__(kSegBlock) k_seg_dot(const SegTable T, const double* __restrict__ a,
-                                                       const double* __restrict__ b, double* out) {
+template <int B>
+__global__ void __launch_bounds__(B) k_seg_dot(const SegTable T, const double* __restrict__ a,
+                                               const double* __restrict__ b, double* out) {
     for (uint32_t c = blockIdx.x; c < T.chunks; c += gridDim.x) {
         double v[1] = {0.0};
 #pragma unroll 4
-        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += kSegBlock) v[0] += a[i] * b[i];
+        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += B) v[0] += a[i] * b[i];
         double* const o[1] = {out};
         seg_store<1>(v, o, T, c);
     }
 }
 
 // vd[s] = Σ v d, dr[s] = Σ d r
-__global__ void __launch_bounds__(kSegBlock) k_seg_dot2(const SegTable T, const double* __restrict__ v,
-                                                        const double* __restrict__ d, const double* __restrict__ r,
-                                                        double* vd, double* dr) {
+template <int B>
+__global__ void __launch_bounds__(B) k_seg_dot2(const SegTable T, const double* __restrict__ v,
+                                                const double* __restrict__ d, const double* __restrict__ r,
+                                                double* vd, double* dr) {
     for (uint32_t c = blockIdx.x; c < T.chunks; c += gridDim.x) {
         double acc[2] = {0.0, 0.0};
 #pragma unroll 4
-        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += kSegBlock) {
+        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += B) {
             acc[0] += v[i] * d[i];
             acc[1] += d[i] * r[i];
         }
@@ -114,18 +116,19 @@ __global__ void __launch_bounds__(kSegBlock) k_seg_dot2(const SegTable T, const 
 }
 
 // active systems: c = (w.v)/(d.v); d = w - c d.  dr[s] = Σ d r (frozen systems keep d)
-__global__ void __launch_bounds__(kSegBlock) k_seg_direction(const SegTable T, const double* __restrict__ w,
-                                                             double* __restrict__ d, const double* __restrict__ r,
-                                                             const double* __restrict__ wv,
-                                                             const double* __restrict__ dv,
-                                                             const int* __restrict__ active, double* dr) {
+template <int B>
+__global__ void __launch_bounds__(B) k_seg_direction(const SegTable T, const double* __restrict__ w,
+                                                     double* __restrict__ d, const double* __restrict__ r,
+                                                     const double* __restrict__ wv,
+                                                     const double* __restrict__ dv,
+                                                     const int* __restrict__ active, double* dr) {
     for (uint32_t k = blockIdx.x; k < T.chunks; k += gridDim.x) {
         const uint32_t s = __ldg(T.seg + k);
         const bool on = active[s] != 0 && dv[s] != 0.0;  // dv = 0: a zero right-hand side, nothing to do
         const double c = on ? wv[s] / dv[s] : 0.0;
         double v[1] = {0.0};
 #pragma unroll 4
-        for (uint32_t i = T.lo[k] + threadIdx.x; i < T.lo[k + 1]; i += kSegBlock) {
+        for (uint32_t i = T.lo[k] + threadIdx.x; i < T.lo[k + 1]; i += B) {
             double di = d[i];
             if (on) {
                 di = w[i] - c * di;
@@ -139,18 +142,19 @@ __global__ void __launch_bounds__(kSegBlock) k_seg_direction(const SegTable T, c
 }
 
 // active systems: a = (d.r)/(d.v); x += a d; r -= a v.  rr[s] = Σ r²
-__global__ void __launch_bounds__(kSegBlock) k_seg_step(const SegTable T, double* __restrict__ x,
-                                                        double* __restrict__ r, const double* __restrict__ d,
-                                                        const double* __restrict__ v, const double* __restrict__ dr,
-                                                        const double* __restrict__ dv, const int* __restrict__ active,
-                                                        double* rr) {
+template <int B>
+__global__ void __launch_bounds__(B) k_seg_step(const SegTable T, double* __restrict__ x,
+                                                double* __restrict__ r, const double* __restrict__ d,
+                                                const double* __restrict__ v, const double* __restrict__ dr,
+                                                const double* __restrict__ dv, const int* __restrict__ active,
+                                                double* rr) {
     for (uint32_t c = blockIdx.x; c < T.chunks; c += gridDim.x) {
         const uint32_t s = __ldg(T.seg + c);
         const bool on = active[s] != 0 && dv[s] != 0.0;
         const double a = on ? dr[s] / dv[s] : 0.0;
         double acc[1] = {0.0};
 #pragma unroll 4
-        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += kSegBlock) {
+        for (uint32_t i = T.lo[c] + threadIdx.x; i < T.lo[c + 1]; i += B) {
             double ri = r[i];
             if (on) {
                 x[i] = x[i] + a * d[i];
@@ -162,6 +166,28 @@ __global__ void __launch_bounds__(kSegBlock) k_seg_step(const SegTable T, double
         double* const o[1] = {rr};
         seg_store<1>(acc, o, T, c);
     }
+}
+
+// The kernels for blocks of `threads` threads.
+struct SegKernels {
+    int threads;
+    decltype(&k_seg_residual<32>) residual;
+    decltype(&k_seg_dot<32>) dot;
+    decltype(&k_seg_dot2<32>) dot2;
+    decltype(&k_seg_direction<32>) direction;
+    decltype(&k_seg_step<32>) step;
+};
+template <int B>
+SegKernels seg_kernels_of() {
+    return {B, k_seg_residual<B>, k_seg_dot<B>, k_seg_dot2<B>, k_seg_direction<B>, k_seg_step<B>};
+}
+// By the rows of a chunk: as many blocks as fill the SMs go over small systems, a few rows a thread
+// (Krylov loop without preconditioner, 12 iterations, us: 20,000 systems of 16 rows 6,340 with 512
+// threads, 4,300 now; 4,096 of 64 rows 1,950, 1,580; 2,000 of 256 rows 1,370, 1,200).
+SegKernels seg_kernels(uint32_t rows) {
+    if (rows <= 64) return seg_kernels_of<32>();
+    if (rows <= 256) return seg_kernels_of<64>();
+    return rows <= 1024 ? seg_kernels_of<256>() : seg_kernels_of<512>();
 }
 
 }  // namespace
@@ -230,7 +256,9 @@ void segmented_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t nseg, co
     double *r = h.r.get(), *wv = h.w.get(), *d = h.d.get(), *v = h.v.get(), *y = h.y.get();
     const SegTable T{w.chunks, w.lo.get(), w.of.get(), w.first.get(), w.partial.get(), w.ticket.get()};
     auto sc = [&](int k) { return w.sc.get() + (size_t)k * nseg; };
-    const int grid = (int)std::min<uint32_t>(w.chunks, (uint32_t)h.info.sms * 4);
+    const SegKernels K = seg_kernels(n / w.chunks);
+    const int per_sm = 2048 / K.threads;
+    const int grid = (int)std::min<uint32_t>(w.chunks, (uint32_t)(h.info.sms * per_sm));
     uint32_t applies = 0, spmvs = 0;
     std::vector<int> act(nseg, 1);
     PRISM_CUDA(cudaMemcpyAsync(w.active.get(), act.data(), nseg * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -238,16 +266,16 @@ void segmented_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t nseg, co
     PRISM_CUDA(cudaEventRecord(h.ev0, s));
     h.spmv(x, y);
     ++spmvs;
-    k_seg_residual<<<grid, kSegBlock, 0, s>>>(T, b, y, r, sc(SG_BB), sc(SG_RES));
+    K.residual<<<grid, K.threads, 0, s>>>(T, b, y, r, sc(SG_BB), sc(SG_RES));
     PRISM_LAUNCHED();
     if (P) { P->apply(s, r, wv); ++applies; }
     else PRISM_CUDA(cudaMemcpyAsync(wv, r, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     PRISM_CUDA(cudaMemcpyAsync(d, wv, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     h.spmv(d, v);
     ++spmvs;
-    k_seg_dot2<<<grid, kSegBlock, 0, s>>>(T, v, d, r, sc(SG_DV), sc(SG_DR));
+    K.dot2<<<grid, K.threads, 0, s>>>(T, v, d, r, sc(SG_DV), sc(SG_DR));
     PRISM_LAUNCHED();
-    k_seg_step<<<grid, kSegBlock, 0, s>>>(T, x, r, d, v, sc(SG_DR), sc(SG_DV), w.active.get(), sc(SG_RR));
+    K.step<<<grid, K.threads, 0, s>>>(T, x, r, d, v, sc(SG_DR), sc(SG_DV), w.active.get(), sc(SG_RR));
     PRISM_LAUNCHED();
     PRISM_CUDA(cudaMemcpyAsync(w.host.data(), w.sc.get(), (size_t)kSegScalars * nseg * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
@@ -291,22 +319,22 @@ void segmented_fcg_solve(Handle& h, const prism_solve_opts& o, uint32_t nseg, co
             PRISM_CUDA(cudaMemcpyAsync(w.active.get(), act.data(), nseg * sizeof(int), cudaMemcpyHostToDevice, s));
         if (flexible && P) { P->apply(s, r, wv); ++applies; }
         else PRISM_CUDA(cudaMemcpyAsync(wv, r, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        k_seg_dot<<<grid, kSegBlock, 0, s>>>(T, wv, v, sc(SG_WV));
+        K.dot<<<grid, K.threads, 0, s>>>(T, wv, v, sc(SG_WV));
         PRISM_LAUNCHED();
-        k_seg_direction<<<grid, kSegBlock, 0, s>>>(T, wv, d, r, sc(SG_WV), sc(SG_DV), w.active.get(),
+        K.direction<<<grid, K.threads, 0, s>>>(T, wv, d, r, sc(SG_WV), sc(SG_DV), w.active.get(),
                                                sc(SG_DR2));
         PRISM_LAUNCHED();
         h.spmv(d, v);
         ++spmvs;
-        k_seg_dot<<<grid, kSegBlock, 0, s>>>(T, v, d, sc(SG_DV));
+        K.dot<<<grid, K.threads, 0, s>>>(T, v, d, sc(SG_DV));
         PRISM_LAUNCHED();
-        k_seg_step<<<grid, kSegBlock, 0, s>>>(T, x, r, d, v, sc(SG_DR2), sc(SG_DV), w.active.get(),
+        K.step<<<grid, K.threads, 0, s>>>(T, x, r, d, v, sc(SG_DR2), sc(SG_DV), w.active.get(),
                                           sc(SG_RR));
         PRISM_LAUNCHED();
     }
     h.spmv(x, y);
     ++spmvs;
-    k_seg_residual<<<grid, kSegBlock, 0, s>>>(T, b, y, nullptr, sc(SG_BB), sc(SG_RES));
+    K.residual<<<grid, K.threads, 0, s>>>(T, b, y, nullptr, sc(SG_BB), sc(SG_RES));
     PRISM_LAUNCHED();
     PRISM_CUDA(cudaEventRecord(h.ev1, s));
     PRISM_CUDA(cudaMemcpyAsync(w.host.data(), w.sc.get(), 2 * (size_t)nseg * sizeof(double), cudaMemcpyDeviceToHost,

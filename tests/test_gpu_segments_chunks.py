@@ -49,3 +49,11 @@ def test_systems_around_a_chunk(seed):
 
 def test_more_chunks_than_blocks():
     solve_all(MANY, 5, [0, 349, 350, 351, 700, 701])
+
+
+@pytest.mark.parametrize("grid,count", [((1, 1), 50), ((8, 8), 60), ((13, 5), 60), ((16, 16), 40), ((19, 14), 40),
+                                        ((32, 32), 12), ((41, 25), 12)])
+def test_sizes_of_blocks(grid, count):
+    """Systems of 1, 64, 65, 256, 266, 1,024 and 1,025 rows: each side of the sizes at which the
+    kernels take larger blocks."""
+    solve_all([grid] * count, 6, [0, count // 2, count - 1])

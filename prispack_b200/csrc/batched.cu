@@ -12,8 +12,9 @@
 // single vector leaves most SMs waiting for it.  The block sweep is the dataflow
 // kernel (flow_sweep.cuh) with 1, 2 or 4 columns a lane: groups of CTAs take the
 // columns, the CTAs of a group the slabs.  (Level order, a warp a row, remains for
-// factors whose slabs do not fit in shared memory; it took 4.2 ms a sweep of IC
-// 192^2 with 64 columns, 0.34 ms now.)
+// factors whose slabs do not fit in shared memory and for blocks it is the faster for
+// (choose_block_sweep); it took 4.2 ms a sweep of IC 192^2 with 64 columns, which now
+// takes 0.31.)
 //
 // Each column follows the recurrence of CG<double>::solve (CG.cpp:34-83) on
 // its own scalars; a column that has converged is frozen (its x and r stop

@@ -186,7 +186,7 @@ static int flow_selftest(uint32_t n, const uint32_t* rowptr, const uint32_t* col
     gather_sweep<Low>(n, rowptr, col, val, diag, op, lower, s);
     prism::FlowLayout L;
     if (!prism::flow_layout<Low>(s, prism::slab_ranges<Low>(s, slabs), max_slots ? max_slots : 0xFFFFu, L))
-        return fail(PRISM_ERR_UNSUPPORTED, "a slab needs more value slots");
+        return fail(PRISM_ERR_UNSUPPORTED, "a slab needs more value slots, or a row more chunks, than there are");
     const std::string why = prism::flow_layout_replay<Low>(s, L, acc32, in, out);
     return why.empty() ? PRISM_OK : fail(PRISM_ERR_ARG, "dataflow layout: " + why);
 }

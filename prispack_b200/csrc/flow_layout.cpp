@@ -184,7 +184,6 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
         const uint32_t nt = (uint32_t)P.chunks.size();
         for (uint32_t w = 0; w < kFlowWorkers; ++w) {
             uint32_t* q = &out.warp[((size_t)b * kFlowWorkers + w) * 8];
-            q[0] = (uint32_t)chunk;
             q[1] = out.tasks;
             q[4] = (uint32_t)(bytes / 16);
             for (uint32_t t = w; t < nt; t += kFlowWorkers) {
@@ -254,7 +253,7 @@ bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32
             for (size_t t = w; t < P.chunks.size(); t += kFlowWorkers, ++task) {
                 const uint32_t nc = P.chunks[t], m = P.task[t + 1] - P.task[t];
                 const size_t tn = t + kFlowWorkers;
-                const uint32_t mn = tn < P.chunks.size() ? (P.task[tn + 1] - P.task[tn]) | (P.chunks[tn] == 1 ? 16u : 0u) : 0u;
+                const uint32_t mn = tn < P.chunks.size() ? P.task[tn + 1] - P.task[tn] : 0u;
                 for (uint32_t j8 = 0; j8 < kFlowRows; ++j8) {
                     uint32_t* h = &out.hdr[((size_t)task * kFlowRows + j8) * 4];
                     h[0] = h[1] = kFlowNone;
@@ -463,7 +462,7 @@ std::string flow_replay(const Sweep<Low>& s, const FlowLayout& L, const double* 
                 ++next[w];
                 if (next[w] < q[2]) {
                     const uint32_t nw = L.hdr[(size_t)(task + 1) * kFlowRows * 4 + 3];
-                    if ((hw >> 12 & 31u) != ((nw >> 8 & 15u) | ((nw & 0xFFu) == 1 ? 16u : 0u))) return "next task";
+                    if ((hw >> 12 & 15u) != (nw >> 8 & 15u)) return "next task";
                 }
                 chunk[w] += nc;
                 at[w] += (uint64_t)nc * m * RB + flow_tail_bytes(m, vb);

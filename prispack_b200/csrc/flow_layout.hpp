@@ -22,16 +22,16 @@
 //            [vb / 4][m] x 16 B, slots [m] x 4 x u16 (padded to 16 B)
 //   hdr      per task and row: {row (kFlowNone: no row), exchange entry its value is
 //            published in (kFlowNone: read by no other slab), slot | barrier << 16,
-//            chunks of the task | m << 8 | m of the worker's next task << 12 | that one has
-//            one chunk << 16 | sync << 17 | arrive << 22}.
+//            chunks of the task | m << 8 | m of the worker's next task << 12 | sync << 17 |
+//            arrive << 22}.
 //            Level l of a slab opens when named barrier 1 + l mod kFlowBars completes, on which
 //            the workers of levels l - 1 and l meet: sync is their number where the task
 //            waits for its level (0: an earlier task of the worker did, or the first
 //            level), arrive that of the next level where the worker is done with this one
 //            and has no task of the next (0 otherwise)
 //   dg       per task and row: the diagonal, or its reciprocal for the dividing operations
-//   warp     per slab and worker: {first chunk, first task, tasks, chunks, start and
-//            length in `chunks` / 16, 0, 0}
+//   warp     per slab and worker: {0, first task, tasks, chunks, start and length in
+//            `chunks` / 16, 0, 0}
 //   halo     per slab, by level: {exchange entry, slot}
 // Slabs are numbered from upstream to downstream.
 #pragma once
@@ -82,8 +82,9 @@ struct FlowLayout {
 };
 
 // Lays the sweep out for slabs [start[b], start[b + 1]), with E = entries (0: by the rows'
-// lengths).  False when a slab needs more than max_slots value slots.  order, coef_map: as for stream_layout (every position is
-// an early one; coef_map in units of the factor value within `chunks`).
+// lengths).  False when a slab needs more than max_slots value slots or a task more than 255 chunks
+// (a row of 4,080 or 8,160 front entries).  order, coef_map: as for stream_layout (every position
+// is an early one; coef_map in units of the factor value within `chunks`).
 template <typename Low>
 bool flow_layout(const Sweep<Low>& s, const std::vector<uint32_t>& start, uint32_t max_slots, FlowLayout& out,
                  StreamOrder* order = nullptr, std::vector<uint32_t>* coef_map = nullptr, uint32_t entries = 0);

@@ -6,15 +6,19 @@
 // What bounds it.  A sweep is a chain of dependency wavefronts, so its time is their
 // number times the latency of one; the bytes would take a tenth of that.  What a warp
 // does once between two wavefronts therefore counts in instructions (4-5 cycles each,
-// dependent), and everything else must happen beside the chain.
+// dependent), and everything else must happen beside the chain.  Where the chain crosses
+// slabs, as on every 3D operator, the hop from one to the next (store, L2, poll, store into
+// the slot, poll: about 1.3 us against 0.12 inside a slab) is most of it: of the 921 us of
+// the level-0 lower sweep of AMSED 128^3 a model of the chain gives 338 to 260 hops and 247 to
+// the rest; the workers' tasks, spread over all of them, would take 144.
 //
 //  - A slab belongs to one CTA at a time and its values to that CTA's shared memory, each
 //    in a slot of its own that holds a sentinel until the value is there.  No slot is used
 //    twice within a slab, so nothing has to be waited for before a write, and a reader
 //    needs no flag.
 //  - kFlowWorkers warps take the tasks in turn.  A task takes a warp some 1,700 cycles, 256
-//    instructions that mostly wait for one another, so every warp counts, and 16 are what
-//    128 registers a thread leave.  13 and three for the halo: IC 512^2 FP64 1,034 us an
+//    instructions that mostly wait for one another, so several must be under way for each
+//    wavefront of a slab, and 16 warps are what 128 registers a thread leave.  13 and three for the halo: IC 512^2 FP64 1,034 us an
 //    apply, FCG with AMSED on 64^3 91.9 ms, FGMRES with GMSLR on 50^3 30.1 ms; 12 and four
 //    1,070, 91.1, 31.3; 14 and two 1,004, 93.5, 29.3.  A warp sums the front of its task, whose
 //    values are mostly there, while the others finish the levels before; the level itself
@@ -69,7 +73,7 @@ PRISM_HD inline uint32_t flow_smem(uint32_t slots, uint32_t ab) { return kFlowFi
 struct FlowArgs {
     const unsigned char* chunks;
     const uint4* hdr;
-    const void* dg;             // Acc per (task, lane)
+    const void* dg;             // Acc per (task, row)
     const uint4* warp;
     const uint32_t* halo_ptr;
     const uint2* halo;

@@ -23,8 +23,6 @@ namespace {
 constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s per dependency wait
 constexpr int kSpmvSubG = 8;                           // lanes per row in k_spmv_sub
 constexpr int kSpmvG = 1, kSpmvU = 2;                  // k_spmv: lanes per row, rows per group and pass
-// the shapes A's SpMV may take (lanes per row, rows per group and pass): one lane per row
-// suits short rows such as stencils, a group of lanes per row longer ones
 // Rows of a dataflow slab the tuner tries.  More slabs share a wavefront's rows among more SMs
 // and let a CTA take its next slab while the wavefront is elsewhere; fewer pay fewer hand-overs
 // from slab to slab (about 1 us each).  Measured (us an M^-1 apply, 512 / 1024 / 2048 / 4096
@@ -38,6 +36,8 @@ constexpr uint32_t kFlowSlabRows[kFlowSizes] = {512, 1024, 2048, 4096};
 // wavefront (512^2, k = 64, 2 columns: 5,266 us with 2,048 rows, 3,047 with 4,096; 192^2: 682 with
 // 1,024, 805 with 2,048).
 static uint32_t block_slab_rows(uint32_t n) { return std::max(1024u, n / 64u); }
+// the shapes A's SpMV may take (lanes per row, rows per group and pass): one lane per row
+// suits short rows such as stencils, a group of lanes per row longer ones
 constexpr int kSpmvShapes = 6;
 constexpr int kSpmvShapeG[kSpmvShapes] = {1, 1, 2, 4, 8, 16};
 constexpr int kSpmvShapeU[kSpmvShapes] = {2, 4, 2, 1, 1, 1};
@@ -152,7 +152,9 @@ static FlowArgs flow_args(const Handle& h, const DevSweep& s, const double* in, 
 // the shortest chain as long as the groups of CTAs that share the slabs are six or more; wider
 // ones read a record for more columns.  Measured (us an IC apply, float values; 1 / 2 / 4
 // columns): 192^2, k = 24: 524 / 560 / 764; 192^2, k = 64: 909 / 682 / 836; 512^2, k = 64:
-// - / 3,047 / 2,672.
+// - / 3,047 / 2,672.  On 3D operators this choice against level order: IC 64^3 FP64, k = 8 / 24 /
+// 64, 1,134 / 2,486 / 3,998 and 16,847 / 17,232 / 10,633; 100^3, k = 64, 14,505 and 18,211 (there
+// choose_block_sweep mixes the two: 12,190).
 uint32_t block_columns(uint32_t k, uint32_t n) { return k <= 24 ? 1u : (n < 131072 ? 2u : 4u); }
 
 void launch_flow_block(const Handle& h, cudaStream_t st, const DevSweep& s, uint32_t k, const double* in, double* out) {

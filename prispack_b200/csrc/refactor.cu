@@ -32,7 +32,9 @@ namespace prism {
 
 namespace {
 constexpr int kRfWarps = kBlock / 32;
-constexpr unsigned long long kRfWaitNs = 1000000000ull;  // 1 s per dependency wait
+// A dependency wait is bounded by 1 s and 20 us for each chunk on the longest chain of columns:
+// columns of a full factor wait for one another's whole work (8 us a chunk, 2.1 s for 1,024 of them).
+constexpr unsigned long long kRfWaitNs = 1000000000ull, kRfChunkNs = 20000ull;
 constexpr uint32_t kRfMaxCol = 1024;                      // longest column a warp holds in shared memory
 
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
@@ -386,6 +388,7 @@ struct RefactorState {
     DevBuf<uint64_t> uo, so;  // per column: its first update entry; its first chunk's segments
     DevBuf<uint16_t> place, seg;  // as RfArgs
     uint32_t smax = 0;
+    unsigned long long wait_ns = kRfWaitNs;
     // the factor values and pivots the sweeps hold, and those a refactorisation writes: swapped
     // where it succeeds, so that one that fails leaves the factor as it was
     DevBuf<float> lt32, lt32_new;
@@ -582,7 +585,8 @@ void TriangularPrecond::refactor() {
         R.smax = P.max_col <= 512 ? 512u : kRfPlace + 1;
         // where each column's update entries start, and the segments of its chunks (cut as RfChunk
         // cuts them); what stands there is found on the device, once
-        std::vector<uint64_t> uo((size_t)P.n + 1, 0), so((size_t)P.n + 1, 0);
+        std::vector<uint64_t> uo((size_t)P.n + 1, 0), so((size_t)P.n + 1, 0), chain((size_t)P.n, 0);
+        uint64_t longest = 0;
         for (uint32_t j = 0; j < P.n; ++j) {
             uint64_t c = 0, chunks = 0, in_chunk = 0;
             uint32_t updates = 32;
@@ -596,10 +600,14 @@ void TriangularPrecond::refactor() {
                 ++updates;
                 in_chunk += one;
                 c += one;
+                chain[j] = std::max(chain[j], chain[P.up_k[u]]);
             }
+            chain[j] += chunks;
+            longest = std::max(longest, chain[j]);
             uo[j + 1] = uo[j] + c;
             so[j + 1] = so[j] + chunks * (F.f0.rowptr[j + 1] - F.f0.rowptr[j] + (ldlt ? 2u : 1u));
         }
+        R.wait_ns = kRfWaitNs + longest * kRfChunkNs;
         R.uo.upload(uo.data(), uo.size(), st);
         R.so.upload(so.data(), so.size(), st);
         // depth of each column in the dependency graph (its updates come from columns k < j),
@@ -660,7 +668,7 @@ void TriangularPrecond::refactor() {
     a.done = R.done.get();
     a.status = R.status.get();
     a.bad_col = R.status.get() + 1;
-    a.wait_ns = kRfWaitNs;
+    a.wait_ns = R.wait_ns;
     if (R.epoch == 0) {  // the products' places, once per pattern
         const size_t ssm = (size_t)kRfWarps * a.max_col * 2 * sizeof(uint32_t);
         PRISM_CUDA(cudaFuncSetAttribute(k_rf_places, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));

@@ -8,6 +8,7 @@ import pytest
 
 import prispack_b200 as P
 from oracle import oracle as orc
+from test_gpu_refactor_chunks import dense
 
 pytestmark = pytest.mark.gpu
 
@@ -49,6 +50,19 @@ def test_longest_columns(n, kind, precision):
         assert np.array_equal(dv, lv)
         if kind == P.PRECOND_ILDLT:
             assert np.array_equal(dd, D)
+
+
+def test_full_factor_of_the_longest_columns():
+    """1,024 columns that wait for one another's whole work: the refactorisation takes longer than
+    a wait without progress may (1 s), and is not given up."""
+    A, val2 = dense(1024, 5)
+    S = P.DeviceSystem(A)
+    S.set_precond(P.PRECOND_IC, tol=1e-14)
+    rp, ci, _, _ = S.precond_factor(0)
+    S.update_values(val2)
+    S.refactor()
+    rc, lv, _ = orc.refactor(P.PRECOND_IC, A.rowptr, A.col, val2, rp, ci, single=False)
+    assert rc == 0 and np.array_equal(S.precond_factor(0)[2], lv)
 
 
 @pytest.mark.parametrize("kind", [P.PRECOND_IC, P.PRECOND_ILDLT])

@@ -64,6 +64,19 @@ def test_columns(matrix, tol, kind, precision):
         columns_match(S, (8, 48, 64))
 
 
+@pytest.mark.parametrize("precision", [P.PRISM_FP64, P.PRISM_FP32])
+@pytest.mark.parametrize("matrix", [random_pattern, lambda: P.CSRMatrix.block_diagonal(
+    [P.CSRMatrix.laplacian(5, 5, 1)] * 3000)[0]])
+def test_columns_of_a_multilevel_preconditioner(matrix, precision):
+    """Levels of a few wide wavefronts; no low-rank terms, so every product is in double."""
+    A = matrix()
+    H = P.HostAmsed(A, precision=precision, levels=3, lanczos_steps=16, low_rank=8, lowrank_type=0, reorder=0)
+    assert not H.info()["ranks"].any()
+    S = P.DeviceSystem(A)
+    S.attach(H)
+    columns_match(S, (1, 8, 40, 64, 8))
+
+
 def test_many_columns_of_a_random_pattern():
     import torch
     A = random_pattern()
